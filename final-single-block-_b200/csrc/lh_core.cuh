@@ -74,7 +74,7 @@ struct Inst {
     double2 *NU1, *NU2, *NU3;                 // Nu of the last substep, rows 1..
     double2 *NXZ1, *NXZ2, *NXZ3;              // x/z part of Nu, rows 1..nyu
     double2 *UVF, *WVF, *VVC;                 // y-flux spectra, rows 0..nyu(+1)
-    double *FACU, *FACV;                      // scaled upper diagonals
+    double *FACU, *FACV;                      // scaled upper diagonals (k_column) or inverse pivots (k_column_tile)
     double2 *PSI;                             // pressure correction, rows 1..nyu
     double2 *Y1, *Y2, *Y3;                    // forward-eliminated rows of a split column pass
     double2 *CARRY;                           // sweep state between its chunks [3][6][nc]

@@ -294,9 +294,18 @@ cudaError_t instance_download(DevInstance &d, double *u1, double *u2, double *u3
 // beside the plane rounds (LH_COLUMN_SPLIT=0/1 overrides).
 constexpr bool kColumnSplitDefault = false;
 
-// Plans with at most this many columns in all use the one-CTA-per-column
-// column pass (LH_SMALL_COLUMNS overrides).
-constexpr long kSmallColumnsDefault = 1536;
+// Lone instances of at most this many columns x rows run the plane pass in one
+// round (plan_build).
+constexpr long kOneRoundRows = 60000;
+
+// Plans of at most this many columns in all run the column pass on tiles
+// (LH_SMALL_COLUMNS overrides): an SM takes 8 columns at a time, so 1184 are one
+// wave of about 5 + 4.5 rows/32 us, against 0.6 us a row of k_column, whatever
+// its columns: three waves from 64 rows on, two below.  Substep on B200, us,
+// k_column / tiles: 2112 columns x 44 rows 58.5 / 56.8, 2664 x 44 111 / 121;
+// 2664 x 97 222 / 216, x 153 343 / 324, x 257 593 / 552; 4704 x 97 174 / 190,
+// x 153 274 / 280, x 257 449 / 442; 28 channels of 144 x 97 185 / 204.
+static long tile_columns(int max_nyu) { return (max_nyu < 64 ? 2 : 3) * 1184L; }
 
 // ---------------------------------------------------------------------------
 namespace {
@@ -464,17 +473,28 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
         // the multi-plane x stage's groups start at absolute planes 1 + kXGroup g,
         // so rounds hold whole groups
         if (fast && xprod_multi(s.Mx) && c >= (size_t)kXGroup) c -= c % kXGroup;
+        // a small instance alone runs one round: two would only double its
+        // launches (16^2 x 44 24.2 -> 22.6 us a substep, x 97 28.8 -> 27.4, 32^2 x
+        // 97 34.2 -> 33.5, x 153 44.6 -> 46.1)
+        if (fast && insts.size() == 1 && insts[q]->inst.chunk >= s.nyu && (long)s.nc * s.nyu <= kOneRoundRows) c = s.nyu;
         chunk_eff[q] = (int)c;
         rounds = std::max(rounds, (s.nyu + chunk_eff[q] - 1) / chunk_eff[q]);
     }
-    // The column pass: with few columns in the plan, one CTA per column with
-    // the rows spread over its lanes (k_column_small); otherwise 32 columns
-    // per CTA, one lane each (k_column).
+    // The column pass: with few columns in the plan, tiles of columns in shared
+    // memory (k_column_tile); otherwise 32 columns per CTA, one lane each
+    // (k_column).
     size_t total_cols = 0;
     for (const DevInstance *d : insts) total_cols += (size_t)d->hs.nc;
+    int max_nyu = 1;
+    for (const DevInstance *d : insts) max_nyu = std::max(max_nyu, d->hs.nyu);
     const char *sc = getenv("LH_SMALL_COLUMNS");
-    const long small_max = sc ? atol(sc) : kSmallColumnsDefault;
-    p.col_small = (long)total_cols <= small_max;
+    const bool tiled = (long)total_cols <= (sc ? atol(sc) : tile_columns(max_nyu));
+    std::vector<int> width(insts.size(), 0);
+    bool sequential = false;
+    for (size_t q = 0; q < insts.size(); q++) {
+        if (tiled) width[q] = column_tile_width(insts[q]->hs.nyu, insts[q]->hs.nc, total_cols);
+        sequential |= width[q] == 0;
+    }
     // Column blocks split over this many back-to-back launches (LH_COLUMN_WAVES):
     // fewer columns in flight keep the pass's intermediates in L2.
     const char *cw = getenv("LH_COLUMN_WAVES");
@@ -529,9 +549,7 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
                 for (int b = 0; b < nbf; b++) L[2][cls_of[q]].push_back({q, j, slot, b, 0});
             }
         }
-        if (p.col_small)
-            for (int c = 0; c < s.nc; c++) p.column.push_back({q, c, 0, 0, 0});
-        else
+        if (width[q] == 0)
             for (int b = 0; b < (s.nc + kColumnThreads - 1) / kColumnThreads; b++) p.column.push_back({q, b, 0, 0, 0});
     }
     std::vector<Work> all;
@@ -557,10 +575,31 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
             }
     p.off_column = all.size();
     all.insert(all.end(), p.column.begin(), p.column.end());
+    p.col_tiles.clear();
+    for (int C : {8, 4, 2}) {
+        Plan::ColLaunch t;
+        t.C = C;
+        t.off = all.size();
+        for (int q = 0; q < (int)insts.size(); q++) {
+            if (width[q] != C) continue;
+            const HostSetup &s = insts[q]->hs;
+            for (int b = 0; b < (s.nc + C - 1) / C; b++) all.push_back({q, b, 0, 0, 0});
+            t.smem = std::max(t.smem, column_tile_smem_bytes(s.nyu, C));
+        }
+        t.count = all.size() - t.off;
+        if (t.count) p.col_tiles.push_back(t);
+    }
+    // LU factors of the tiled instances, both grids
+    p.off_factors = all.size();
+    for (int q = 0; q < (int)insts.size(); q++)
+        if (width[q] != 0)
+            for (int b = 0; b < (insts[q]->hs.nc + kFactorColumns - 1) / kFactorColumns; b++)
+                for (int grid = 0; grid < 2; grid++) all.push_back({q, b, 0, grid, 0});
+    p.n_factors = all.size() - p.off_factors;
     // split column pass: per round, every instance's rows of that round x its
     // column blocks; plus one chunk of all rows
     const char *cs = getenv("LH_COLUMN_SPLIT");
-    p.col_split = !p.col_small && (cs ? cs[0] == '1' : kColumnSplitDefault);
+    p.col_split = p.col_tiles.empty() && (cs ? cs[0] == '1' : kColumnSplitDefault);
     p.col_a.assign(rounds, {0, 0});
     p.off_col_full = p.n_col_full = 0;
     if (p.col_split) {
@@ -591,6 +630,11 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
             e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
             if (e == cudaSuccess) p.ev_round.push_back(ev);
         }
+        if (e != cudaSuccess) return e;
+    }
+    if (p.n_factors) {
+        if (!p.side_f && rounds > 1) e = cudaStreamCreateWithFlags(&p.side_f, cudaStreamNonBlocking);
+        if (e == cudaSuccess && !p.ev_f) e = cudaEventCreateWithFlags(&p.ev_f, cudaEventDisableTiming);
         if (e != cudaSuccess) return e;
     }
     if (!p.ev_fork) e = cudaEventCreateWithFlags(&p.ev_fork, cudaEventDisableTiming);
@@ -628,12 +672,10 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
     if (gz && (e = raise_smem_limit((const void *)k_zinv, gz)) != cudaSuccess) return e;
     if (gx && (e = raise_smem_limit((const void *)k_xprod, gx)) != cudaSuccess) return e;
     if (gf && (e = raise_smem_limit((const void *)k_zfwd, gf)) != cudaSuccess) return e;
-    int max_nyu = 1;
-    for (const DevInstance *d : insts) max_nyu = std::max(max_nyu, d->hs.nyu);
-    if (p.col_small) {
-        p.sm_col = column_small_smem_bytes(max_nyu);
-        return raise_smem_limit((const void *)k_column_small, p.sm_col);
-    }
+    p.sm_factors = 3 * (size_t)(max_nyu + 1) * sizeof(double);
+    for (const Plan::ColLaunch &t : p.col_tiles)
+        if ((e = column_tile_attributes(t.C, t.smem)) != cudaSuccess) return e;
+    if (!sequential) return cudaSuccess;
     p.sm_col = column_smem_bytes(max_nyu);
     if ((e = raise_smem_limit((const void *)k_column_a, p.sm_col)) != cudaSuccess) return e;
     if ((e = raise_smem_limit((const void *)k_column_bcd, p.sm_col)) != cudaSuccess) return e;
@@ -658,6 +700,10 @@ void plan_free(Plan &p)
     p.ev_round.clear();
     if (p.ev_a) cudaEventDestroy(p.ev_a);
     p.ev_a = nullptr;
+    if (p.ev_f) cudaEventDestroy(p.ev_f);
+    p.ev_f = nullptr;
+    if (p.side_f) cudaStreamDestroy(p.side_f);
+    p.side_f = nullptr;
     if (p.side_a) cudaStreamDestroy(p.side_a);
     p.side_a = nullptr;
 }
@@ -709,6 +755,16 @@ cudaError_t launch_substep(const Plan &p, const Inst *d_insts, int kRK, bool cfl
         if (nstreams <= 1 && (e = cudaEventRecord(p.ev_fork, st)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(p.side_a, p.ev_fork, 0)) != cudaSuccess) return e;
     }
+    // the tiles' LU factors beside the plane pass too, unless dt is only known
+    // after it
+    const bool f_beside = p.n_factors && !(kRK == 1 && cfl_any) && timer == nullptr;
+    if (f_beside) {
+        if (nstreams <= 1 && !a_stream && (e = cudaEventRecord(p.ev_fork, st)) != cudaSuccess) return e;
+        cudaStream_t sf = p.rounds.size() > 1 ? p.side_f : p.side[0];  // a lone round leaves the side stream free
+        if ((e = cudaStreamWaitEvent(sf, p.ev_fork, 0)) != cudaSuccess) return e;
+        factors_launch((unsigned)p.n_factors, p.sm_factors, sf, d_insts, p.d_work + p.off_factors, kRK);
+        if ((e = cudaEventRecord(p.ev_f, sf)) != cudaSuccess) return e;
+    }
     for (size_t ri = 0; ri < p.rounds.size(); ri++) {
         for (const Group &g : p.rounds[ri]) {
             const Work *w = p.d_work + g.off;
@@ -759,15 +815,20 @@ cudaError_t launch_substep(const Plan &p, const Inst *d_insts, int kRK, bool cfl
         if ((e = time_end(timer, 3, st)) != cudaSuccess) return e;
     }
     if (before_column && (e = cudaStreamWaitEvent(st, before_column, cudaEventWaitExternal)) != cudaSuccess) return e;
+    if (f_beside && (e = cudaStreamWaitEvent(st, p.ev_f, 0)) != cudaSuccess) return e;
+    if (p.n_factors && !f_beside) {
+        time_begin(timer, st);
+        factors_launch((unsigned)p.n_factors, p.sm_factors, st, d_insts, p.d_work + p.off_factors, kRK);
+        if ((e = time_end(timer, 3, st)) != cudaSuccess) return e;
+    }
     time_begin(timer, st);
     if (p.col_split) {
         if (!a_beside)
             k_column_a<<<(unsigned)p.n_col_full, kColumnBlock, p.sm_col, st>>>(d_insts, p.d_work + p.off_col_full, kRK);
         k_column_bcd<<<(unsigned)p.column.size(), kColumnBlock, p.sm_col, st>>>(d_insts, p.d_work + p.off_column, kRK);
-    } else if (p.col_small)
-        k_column_small<<<(unsigned)p.column.size(), 32 * kSmallWarps, p.sm_col, st>>>(d_insts, p.d_work + p.off_column,
-                                                                                      kRK);
-    else {
+    } else {
+        for (const Plan::ColLaunch &t : p.col_tiles)
+            column_tile_launch(t.C, (unsigned)t.count, t.smem, st, d_insts, p.d_work + t.off, kRK);
         const size_t nb = p.column.size(), per = (nb + p.col_waves - 1) / p.col_waves;
         for (size_t b0 = 0; b0 < nb; b0 += per)
             k_column<<<(unsigned)std::min(per, nb - b0), kColumnBlock, p.sm_col, st>>>(

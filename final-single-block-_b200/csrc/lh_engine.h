@@ -100,7 +100,16 @@ struct Plan {
     size_t work_cap = 0;     // Work entries d_work holds (reused across rebuilds)
     size_t off_column = 0;
     size_t sm_col = 0;
-    bool col_small = false;  // column pass by k_column_small (one CTA per column)
+    // column pass on tiles of C columns (k_column_tile), one launch per width
+    struct ColLaunch {
+        int C = 0;
+        size_t off = 0, count = 0, smem = 0;
+    };
+    std::vector<ColLaunch> col_tiles;
+    size_t off_factors = 0, n_factors = 0, sm_factors = 0;  // their LU factors (k_factors), beside the plane pass
+    // (on side_f, or on side[0] when there is one round)
+    cudaStream_t side_f = nullptr;
+    cudaEvent_t ev_f = nullptr;
     int col_waves = 1;       // column-pass launches the column blocks are split over
     // Split column pass (LH_COLUMN_SPLIT): its forward sweeps run in row
     // chunks, one per plane round, on a stream of their own as soon as the

@@ -8,12 +8,14 @@ namespace lh {
 constexpr int kColumnThreads = 32;       // columns per column-pass CTA (one lane each)
 constexpr int kColumnBlock = 3 * kColumnThreads;  // three warps: the u1, u3 and u2 chains
 size_t column_smem_bytes(int max_nyu);  // ring + staged y metrics
-// column pass for small mode counts: one CTA of kSmallWarps warps (the u1,
-// u3, u2 chains) per column, rows spread over the lanes
-constexpr int kSmallWarps = 3;
-// rows per lane whose global loads the right-hand-side phase issues together
-constexpr int kSmallBatch = 4;
-size_t column_small_smem_bytes(int max_nyu);
+// column pass on tiles in shared memory (lh_column_tile.cu)
+int column_tile_width(int nyu, int nc, size_t total);  // columns per tile of an instance, 0: not served
+size_t column_tile_smem_bytes(int nyu, int C);
+cudaError_t column_tile_attributes(int C, size_t smem);
+void column_tile_launch(int C, unsigned grid, size_t smem, cudaStream_t st, const Inst *insts, const Work *work, int kRK);
+// the tiles' inverse pivots into FACU / FACV, before column_tile_launch
+constexpr int kFactorColumns = 8, kFactorBlocks = 32;  // columns and lanes per column of a k_factors CTA
+void factors_launch(unsigned grid, size_t smem, cudaStream_t st, const Inst *insts, const Work *work, int kRK);
 
 __global__ void k_zinv(const Inst *__restrict__ insts, const Work *__restrict__ work, int bc);
 __global__ void k_xprod(const Inst *__restrict__ insts, const Work *__restrict__ work, int br, int want_max);
@@ -31,7 +33,6 @@ __global__ void k_column_bcd(const Inst *__restrict__ insts, const Work *__restr
 __global__ void k_dt(const Inst *__restrict__ insts, int ninst);
 __global__ void k_col_to_plane(const double2 *__restrict__ src, double2 *__restrict__ dst, int len, int nc);
 __global__ void k_plane_to_col(const double2 *__restrict__ src, double2 *__restrict__ dst, int len, int nc);
-__global__ void k_column_small(const Inst *__restrict__ insts, const Work *__restrict__ work, int kRK);
 __global__ void k_lusolu(const Inst *__restrict__ insts, int grid, int kRK, double dt, const double2 *rhs,
                          double2 *u, double *fac);
 __global__ void k_lusolp(const Inst *__restrict__ insts, double2 *x);

@@ -1,0 +1,47 @@
+"""The column pass on shared-memory tiles against the sequential one, at the
+sizes where a tile can go wrong: column counts that are no multiple of the tile
+width (2, 4 and 8 columns), fewer rows than the 32 row blocks, rows that fill
+the blocks exactly or leave the last ones empty, tall columns, constant flow
+rate (its exact block entries) and the CFL time step."""
+import pytest
+
+from helpers import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# Nx, Nz, ny, constant pressure gradient, CFL: the tile is 2 columns wide up to
+# 296 columns, 4 up to 1184, 8 above
+SIZES = [
+    (16, 4, 5, 1, False),      # 36 columns, 4 rows on 32 blocks
+    (8, 18, 33, 0, False),     # 90 columns, 32 rows
+    (32, 18, 34, 1, True),     # 306 columns: a half-filled last tile; one row more than blocks
+    (32, 18, 65, 0, False),    # 64 rows, two to a block
+    (64, 36, 66, 1, False),    # 1188 columns: 4 live in the last tile
+    (64, 36, 129, 0, False),
+    (64, 36, 401, 1, False),   # tall columns: shared memory narrows the tile
+]
+
+
+@pytest.mark.parametrize("Nx,Nz,ny,ctpress,cfl", SIZES)
+def test_tiles_match_the_sequential_pass(Nx, Nz, ny, ctpress, cfl, monkeypatch):
+    """Only the values entering a block of rows are formed in another order:
+    the bounds of the per-column pass hold (1e-13, p 1e-12)."""
+    from lh_b200 import Desc, Engine, grids, perturbed_laminar
+    d = Desc(Nx=Nx, Nz=Nz, ny=ny, flag_ctpress=ctpress, dt_mode=0 if cfl else 1, dt=1e-3, CFL=0.5)
+    ic = perturbed_laminar(d, 31, *grids(d))
+    out = []
+    for limit in ("0", "1000000000"):
+        monkeypatch.setenv("LH_SMALL_COLUMNS", limit)
+        e = Engine(d)
+        e.upload(*ic)
+        e.step(2)
+        e.synchronize()
+        out.append((e.download(), e.scalars(), e.error_div()))
+        e.close()
+    for f in ("u1", "u2", "u3", "p"):
+        assert rel_l2(out[1][0][f], out[0][0][f]) <= (1e-12 if f == "p" else 1e-13), f
+    assert out[0][1]["iter"] == out[1][1]["iter"] == 2
+    for k in ("t", "Qx", "mpgx"):
+        # mpgx: a flow-rate difference over dt; its terms agree to the last bit
+        assert abs(out[1][1][k] - out[0][1][k]) <= 1e-10 * abs(out[0][1][k]), k
+    assert out[1][2] < 1e-11
