@@ -334,12 +334,9 @@ ClassTiles fast_tiles(const HostSetup &s, int cbz_max, int rb, int cbf_max)
     c.cbz = (s.nxh + nb - 1) / nb;
     c.tz = fast_threads(s.Mz, c.cbz);
     c.smz = zinv_smem(s.Mz, c.cbz);
-    rb = std::max(1, std::min(rb, s.Mz));
-    // the x stage's vectors sit at an odd row stride (3 rb rounded up to odd)
-    while (rb > 1 && !(xprod_threads(s.Mx, rb) <= xprod_max_threads(s.Mx) && xprod_smem(s.Mx, rb) <= smax)) rb--;
-    c.rbx = rb;
-    c.tx = xprod_threads(s.Mx, rb);
-    c.smx = xprod_smem(s.Mx, rb);
+    c.rbx = xprod_rows(s.Mx, std::max(1, std::min(rb, s.Mz)));
+    c.tx = xprod_threads(s.Mx, c.rbx);
+    c.smx = xprod_smem(s.Mx, c.rbx);
     cbf_max = std::max(1, std::min(cbf_max, s.nxh));
     // z forward: one half of the six products (3 vectors per x mode) per CTA
     while (cbf_max > 1 && !(zfwd_threads(s.Mz, cbf_max) <= fast_max_threads(2) && zfwd_smem(s.Mz, cbf_max) <= smax))
@@ -352,20 +349,16 @@ ClassTiles fast_tiles(const HostSetup &s, int cbz_max, int rb, int cbf_max)
 }
 
 // Default tile bounds of a fast size: measured on B200 at 128^2 (16 threads
-// per vector): 16 x modes per z-inverse CTA, 4 z rows per x CTA, up to 4 x
-// modes per z-forward CTA; sizes with fewer threads per vector take
-// proportionally more, the x stage at 18 and more one z row.  The z-forward bound is 80/vz, one less at Mz = 96
-// and 192 (ny = 153 sweeps: one x mode fewer was faster there, slower at
-// Mz = 288 and 384, even at 48).
+// per vector): 16 x modes per z-inverse CTA, up to 4 x modes per z-forward CTA;
+// sizes with fewer threads per vector take proportionally more.  The z-forward
+// bound is 80/vz, one less at Mz = 96 and 192 (ny = 153 sweeps: one x mode fewer
+// was faster there, slower at Mz = 288 and 384, even at 48).  The x stage takes
+// whole CTAs of four warps; 2 to 32 rows per CTA made no difference.
 void default_bounds(const HostSetup &s, int &cbz, int &rbx, int &cbf)
 {
-    const int vz = std::max(1, fast_vector_threads(s.Mz)), vx = std::max(1, fast_vector_threads(s.Mx));
+    const int vz = std::max(1, fast_vector_threads(s.Mz));
     cbz = 256 / vz;
-    // the multi-plane x stage holds seven vectors per z row: one row group;
-    // the block-synchronous stage at 18 and 24 threads per vector (Ngal 288,
-    // 384) is fastest with one z row per CTA (autotuner on B200: 192^2 x 257
-    // 5.43 -> 5.07 ms per step, 256^2 x 257 10.11 -> 9.76)
-    rbx = vx >= 18 && !xprod_warp(s.Mx) ? 1 : std::max(1, (xprod_multi(s.Mx) ? 32 : 64) / vx);
+    rbx = xprod_rows(s.Mx, s.Mz);
     cbf = std::max(1, 80 / vz - ((s.Mz == 96 || s.Mz == 192) ? 1 : 0));
 }
 
@@ -470,9 +463,6 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
         size_t c = fast ? (units > fixed ? (units - fixed) / 9 : kRoundStreams) : units / kNumProducts;
         c = std::max<size_t>(c / kRoundStreams, (size_t)(s.nyu + 7) / 8);
         c = std::max<size_t>(1, std::min<size_t>(c, (size_t)insts[q]->inst.chunk / kRoundStreams));
-        // the multi-plane x stage's groups start at absolute planes 1 + kXGroup g,
-        // so rounds hold whole groups
-        if (fast && xprod_multi(s.Mx) && c >= (size_t)kXGroup) c -= c % kXGroup;
         // a small instance alone runs one round: two would only double its
         // launches (16^2 x 44 24.2 -> 22.6 us a substep, x 97 28.8 -> 27.4, 32^2 x
         // 97 34.2 -> 33.5, x 153 44.6 -> 46.1)
@@ -526,15 +516,8 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
                         for (int b = 0; b < nbz; b++)
                             L[0][cls_of[q]].push_back({q, jp, sb + jp - j0 + 1, f * nbz + b, 0});
                     }
-                if (xprod_multi(s.Mx))
-                    for (int j = j0; j <= j1; j += kXGroup) {
-                        const int np = std::min(kXGroup, j1 - j + 1);
-                        for (int b = 0; b < nbx; b++)
-                            L[1][cls_of[q]].push_back({q, j, pb + j - j0, b | (np << 16), sb + j - j0});
-                    }
                 for (int j = j0; j <= j1; j++) {
-                    if (!xprod_multi(s.Mx))
-                        for (int b = 0; b < nbx; b++) L[1][cls_of[q]].push_back({q, j, pb + j - j0, b, sb + j - j0});
+                    for (int b = 0; b < nbx; b++) L[1][cls_of[q]].push_back({q, j, pb + j - j0, b, sb + j - j0});
                     for (int b = 0; b < nbf; b++)
                         for (int h = 0; h < 2; h++) L[2][cls_of[q]].push_back({q, j, pb + j - j0, 2 * b + h, 0});
                 }

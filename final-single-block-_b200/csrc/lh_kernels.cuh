@@ -49,12 +49,10 @@ cudaError_t raise_smem_limit(const void *func, size_t bytes);
 // compile-time-sized fast path (lh_plane_fast.cu)
 bool fast_size(int n);
 int fast_threads(int n, int vectors);
-int fast_max_threads(int stage);  // launch-bounds block size of a fast stage
+int fast_max_threads(int stage);  // launch-bounds block size of a z stage
 int fast_vector_threads(int n);   // threads per vector of a fast length
 size_t zinv_smem(int n, int cb);  // shared memory of a z-inverse CTA of cb vectors
-bool xprod_warp(int n);            // the x stage of length n runs a warp-local kernel
-bool xprod_multi(int n);           // the x stage of length n runs the multi-plane kernel
-int xprod_max_threads(int n);      // launch-bounds block size of that x-stage kernel
+int xprod_rows(int n, int rb);     // z rows per CTA the kernel takes for a bound rb
 int xprod_threads(int n, int rb);  // threads of an x-stage CTA of rb z rows
 size_t xprod_smem(int n, int rb);  // shared memory of an x-stage CTA of rb z rows
 int zfwd_threads(int n, int cb);   // threads of a z-forward CTA of cb x modes

@@ -16,6 +16,7 @@
 // 373-418) are linear and commute with the z transform, so they are applied
 // to the z-transformed rows in the x stage: the z inverse runs on three
 // fields per plane instead of six.
+#include <algorithm>
 #include <cstdlib>
 
 #include "lh_fft.cuh"
@@ -30,18 +31,6 @@
 #endif
 #ifndef LH_ZINV_B
 #define LH_ZINV_B 3
-#endif
-#ifndef LH_XPROD_T
-#define LH_XPROD_T 256
-#endif
-#ifndef LH_XPROD_B
-#define LH_XPROD_B 3
-#endif
-#ifndef LH_XMULTI_T
-#define LH_XMULTI_T 192
-#endif
-#ifndef LH_XMULTI_B
-#define LH_XMULTI_B 2
 #endif
 #ifndef LH_ZFWD_T
 #define LH_ZFWD_T 256
@@ -63,14 +52,11 @@
 #define LH_LARGE_B 2
 #endif
 #define LH_MINB(N, B) ((N) >= LH_LARGE_N ? LH_LARGE_B : (B))
-// iterations of the warp-local x stage's gather loop unrolled (its loads of
-// later modes are then issued before the shared-memory stores of earlier ones)
-#ifndef LH_XGATHER_UNROLL
-#define LH_XGATHER_UNROLL 1
-#endif
 #include "lh_kernels.cuh"
 
 namespace lh {
+
+constexpr int kXprodThreads = 128;  // most threads of a k_xprod_r CTA
 
 // Outer twiddles W^(r k1), k1 = 1.., of a two-pass transform by the
 // recurrence W^(r k1) = W^(r (k1-1)) W^r from one table entry, which keeps the
@@ -215,643 +201,238 @@ __global__ void __launch_bounds__(LH_ZINV_T, LH_ZINV_B) k_zinv_w(const Inst *__r
 }
 
 // ---------------------------------------------------------------------------
-// x transforms and products of one (plane j, block of rb z rows).  Rows are
-// gathered from Sin with the y interpolations (interp_v FOU3D.f90:407,
-// interp_u :387): fields 0 u1(j), 1 u2 at centre j, 2 u3(j), 3 u1 at face j,
-// 4 u2(j), 5 u3 at face j; then inverse real x FFT (two real rows per
-// complex FFT), products, forward real x FFT (ops_in_planes2,
-// FOU3D.f90:1514-1652) -> Sprod[slot]
+// x transforms and products of one (plane j, block of z rows), the products in
+// registers.  N1 lanes of a warp own a z row and take its three vectors (pairs)
+// in turn; NX = N1 N2.
+//
+//   gather   the lane of task n2 loads the modes k = n2 + N2 q <= Nx/2 of the
+//            pair's two real rows A, B (with the y interpolations), forms z[k] =
+//            A + iB for itself and z[NX - k] = conj(A) + i conj(B) for the lane
+//            of task N2 - n2 (one shuffle), so the inputs of the inverse
+//            transform never pass through shared memory;
+//   inverse  DFT over N1, twiddle, exchange through the row's N1 x N2 matrix,
+//            DFT over N2: lane r holds the physical values x = r + N1 t;
+//   products in registers: u3^2 of the first pair waits for the second, u2 of
+//            the second for the third;
+//   forward  the mirrored split (DFT over N2 first, in the registers that hold
+//            the products), exchange, DFT over N1: the lane of task m holds the
+//            modes k = m + N2 q;
+//   split    the packed real transforms need Z[NX - k], on the lane of task
+//            N2 - m: one shuffle again; modes i <= Nx/2 are stored.
+//
+// A vector crosses shared memory twice (the exchanges, 4 accesses an element)
+// instead of 12 accesses when the gather, the products and the split went
+// through it too, which kept that pipe busier than the FP64 pipe.  Tasks come in
+// rounds of N1 whose sets are closed under m -> N2 - m, and a lane keeps its
+// columns of the matrix from one use to the next, so two __syncwarp a vector are
+// all the synchronisation.  Every load of a task is issued before the first is
+// used: loaded mode by mode the stage waited on L2 for half its time.
+//
+// What bounds it: the FP64 pipe, 48 % busy (55 % on the busiest SM), at the
+// warps that 168 registers leave (three CTAs of 128); then the L2 gather and the
+// launch's last wave.  x products alone, us a substep on B200, before (one
+// vector a half warp, or block-synchronous where vectors do not fit a warp) ->
+// now: 64^2 x 153 72 -> 61, 128^2 x 153 231 -> 183, 192^2 x 257 958 -> 900, 256^2
+// x 257 1955 -> 1340; the substep 128 -> 114, 401 -> 362, 1639 -> 1548, 3258 -> 2695.
+// Four CTAs an SM (128 registers) spill: 372 us at 128^2, 1764 at 192^2; three
+// instead of two at Mx = 384 3150.
 template <int NX>
-__global__ void __launch_bounds__(LH_XPROD_T, LH_MINB(NX, LH_XPROD_B)) k_xprod_f(const Inst *__restrict__ insts, const Work *__restrict__ work,
-                                                          int count, int rb, int want_max)
+struct XPlan {
+    // the substep at the other splits, us: 192 as 8 x 24 394 (16 x 12: 362), 144 as
+    // 8 x 18 153 (148), 96 as 4 x 24 129 and 16 x 6 123 (114), 48 as 4 x 12 51 (44)
+    static constexpr int N1 = NX == 12 ? 4 : (NX <= 96 ? 8 : 16);
+    static constexpr int N2 = NX / N1;
+    static constexpr int LD = N2 | 1;             // odd row stride: conflict-free rows and columns
+    static constexpr int KQ = NX / 3 / N2 + 1;    // modes k <= Nx/2 of a task, at most
+    static constexpr int ROUNDS = N2 <= N1 ? 1 : ((N2 + 1) / 2 + N1 / 2 - 1) / (N1 / 2);
+    static constexpr int RW = 32 / N1;            // rows per warp
+};
+// Task of lane r in round g and the lane that holds task N2 - m; -1: idle.
+// Round 0: m = 0 .. N1/2 - 1, N2/2, and the mirror images N2 - m downwards from
+// the last lane; round g: m = N1/2 g + .. and its mirror images.
+template <int N1, int N2>
+__device__ __forceinline__ void xtask(int g, int r, int &m, int &partner)
 {
-    constexpr int N1 = Plan2<NX>::N1, N2 = Plan2<NX>::N2;
-    extern __shared__ double2 sm[];
-    __shared__ double red[2][16];
-    double2 *buf = sm;
-    if ((int)blockIdx.x >= count) return;
-    const double2 *tw = insts[work[blockIdx.x].inst].twx;  // depends on Mx only
-    // buf[x][v] with an odd row stride ld (double2): the column-wise gather
-    // and pass-2 accesses then spread over all bank groups
-    const int t = threadIdx.x, nv = 3 * rb, ld = nv | 1, v = t % nv, r = t / nv;
-    const double2 twr = __ldg(tw + r);  // outer-twiddle base W^r, issued before the data loads
-    constexpr int nxh = NX / 3 + 1;  // Nx/2 + 1 with Mx = 3 Nx / 2
-    const FastDiv by_rb(rb), by_nv(nv);
-    {
-        const Work w = work[blockIdx.x];
-        const Inst &I = insts[w.inst];
-        const int Mz = I.Mz, j = w.j;
-        const int q0 = w.blk * rb;
-        const size_t fs = (size_t)Mz * nxh;
-        const double2 *u1j = sin_field(I, w.aux + 1, 0), *u3j = u1j + fs, *vj = u3j + fs;
-        const double2 *vjm = sin_field(I, w.aux, 2);
-        const double2 *u1p = sin_field(I, w.aux + 2, 0), *u3p = u1p + fs;
-        const double dnv = 1.0 / (I.yv[j] - I.yv[j - 1]), dnu = 1.0 / (I.yu[j + 1] - I.yu[j]);
-        const double w0v = (I.yu[j] - I.yv[j - 1]) * dnv, w1v = (I.yv[j] - I.yu[j]) * dnv;
-        const double w0u = (I.yv[j] - I.yu[j]) * dnu, w1u = (I.yu[j + 1] - I.yv[j]) * dnu;
-        double2 *S = sprod_slot(I, w.slot);
-        // (0) coalesced gather of the rows (k fastest) straight into the packed
-        // complex vectors of the inverse transform, z[n][v] (v = pair*rb + row):
-        // z = A + iB for the two real rows A, B of a pair, Hermitian-extended,
-        // Im of mode 0 dropped (rft_buff.f:78-81), zero between the retained
-        // modes
-        for (int e = t; e < 3 * rb * nxh; e += blockDim.x) {
-            const int fr = e / nxh, k = e - fr * nxh, p2 = by_rb.div(fr), r2 = by_rb.mod(fr, p2);
-            const int q = q0 + r2;
-            double2 A = make_double2(0.0, 0.0), B = A;
-            if (q < Mz) {
-                const size_t o = (size_t)q * nxh + k;
-                if (p2 == 0) {  // (u1, u3) at the centre
-                    A = u1j[o];
-                    B = u3j[o];
-                } else if (p2 == 1) {  // (u2 at the centre, u2 at the face)
-                    const double2 x0 = vj[o], x1 = vjm[o];
-                    A = make_double2(w0v * x0.x + w1v * x1.x, w0v * x0.y + w1v * x1.y);
-                    B = x0;
-                } else {  // (u1, u3) at the face
-                    const double2 a0 = u1p[o], a1 = u1j[o], b0 = u3p[o], b1 = u3j[o];
-                    A = make_double2(w0u * a0.x + w1u * a1.x, w0u * a0.y + w1u * a1.y);
-                    B = make_double2(w0u * b0.x + w1u * b1.x, w0u * b0.y + w1u * b1.y);
-                }
-            }
-            const int vv = p2 * rb + r2;
-            if (k == 0) {
-                buf[vv] = make_double2(A.x, B.x);
-            } else {
-                buf[k * ld + vv] = make_double2(A.x - B.y, A.y + B.x);
-                buf[(NX - k) * ld + vv] = make_double2(A.x + B.y, B.x - A.y);
-            }
-        }
-        for (int e = t; e < (NX - 2 * nxh + 1) * nv; e += blockDim.x) {
-            const int x = by_nv.div(e);
-            buf[(nxh + x) * ld + by_nv.mod(e, x)] = make_double2(0.0, 0.0);
-        }
-        __syncthreads();
-        // (1) inverse pass 1: lane r < N2 holds n = r + N2*n1
-        {
-            double2 a[N1];
-            if (r < N2) {
-#pragma unroll
-                for (int n1 = 0; n1 < N1; n1++) a[n1] = buf[(r + N2 * n1) * ld + v];
-            }
-            __syncthreads();
-            if (r < N2) {
-                DFT<N1, +1, NX>::run(a, tw);
-                TwStep ts(twr);
-#pragma unroll
-                for (int k1 = 0; k1 < N1; k1++) {
-                    double2 z = a[k1];
-                    if (k1 > 0) z = twiddle<+1>(ts.next(), z);
-                    buf[(k1 * N2 + r) * ld + v] = z;
-                }
-            }
-        }
-        __syncthreads();
-        // (2) inverse pass 2 -> physical values buf[x][v]
-        {
-            double2 b[N2];
-            if (r < N1) {
-#pragma unroll
-                for (int n2 = 0; n2 < N2; n2++) b[n2] = buf[(r * N2 + n2) * ld + v];
-                DFT<N2, +1, NX>::run(b, tw);
-            }
-            __syncthreads();
-            if (r < N1) {
-#pragma unroll
-                for (int k2 = 0; k2 < N2; k2++) buf[(r + N1 * k2) * ld + v] = b[k2];
-            }
-        }
-        __syncthreads();
-        // (3) products; CFL maxima over planes 1..nyu-1 (dtc_calc's dummies see
-        // actual planes 0..nyu-1, FOU3D.f90:622-626)
-        const bool track = want_max && I.dt_mode == 0 && j <= I.nyu - 1;
-        double m1 = 0.0, m3 = 0.0;
-        for (int e = t; e < NX * rb; e += blockDim.x) {
-            const int x = by_rb.div(e), r2 = by_rb.mod(e, x);
-            double2 *p = buf + x * ld;
-            const double2 p0 = p[r2], p1 = p[rb + r2], p2 = p[2 * rb + r2];
-            const double u1 = p0.x, u3 = p0.y, u2c = p1.x, u2 = p1.y, u1f = p2.x, u3f = p2.y;
-            if (track && q0 + r2 < Mz) {
-                m1 = fmax(m1, fabs(u1));
-                m3 = fmax(m3, fabs(u3));
-            }
-            p[r2] = make_double2(u1 * u1, u1 * u3);
-            p[rb + r2] = make_double2(u2c * u2c, u3 * u3);
-            p[2 * rb + r2] = make_double2(u1f * u2, u3f * u2);
-        }
-        if (track) {
-            for (int o = 16; o > 0; o >>= 1) {
-                m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-                m3 = fmax(m3, __shfl_xor_sync(0xffffffffu, m3, o));
-            }
-            if ((t & 31) == 0) {
-                red[0][t >> 5] = m1;
-                red[1][t >> 5] = m3;
-            }
-        }
-        __syncthreads();
-        if (track && t == 0) {
-            double a1 = 0.0, a3 = 0.0;
-            for (int k = 0; k < (int)(blockDim.x + 31) / 32; k++) {
-                a1 = fmax(a1, red[0][k]);
-                a3 = fmax(a3, red[1][k]);
-            }
-            atomicMax(reinterpret_cast<unsigned long long *>(&I.sc[SC_U1MAX]), (unsigned long long)__double_as_longlong(a1));
-            atomicMax(reinterpret_cast<unsigned long long *>(&I.sc[SC_U3MAX]), (unsigned long long)__double_as_longlong(a3));
-        }
-        // (4) forward pass 1
-        {
-            double2 a[N1];
-            if (r < N2) {
-#pragma unroll
-                for (int n1 = 0; n1 < N1; n1++) a[n1] = buf[(r + N2 * n1) * ld + v];
-                DFT<N1, -1, NX>::run(a, tw);
-            }
-            __syncthreads();
-            if (r < N2) {
-                TwStep ts(twr);
-#pragma unroll
-                for (int k1 = 0; k1 < N1; k1++) {
-                    double2 z = a[k1];
-                    if (k1 > 0) z = twiddle<-1>(ts.next(), z);
-                    buf[(k1 * N2 + r) * ld + v] = z;
-                }
-            }
-        }
-        __syncthreads();
-        // (5) forward pass 2 -> X[k][v]
-        {
-            double2 b[N2];
-            if (r < N1) {
-#pragma unroll
-                for (int n2 = 0; n2 < N2; n2++) b[n2] = buf[(r * N2 + n2) * ld + v];
-                DFT<N2, -1, NX>::run(b, tw);
-            }
-            __syncthreads();
-            if (r < N1) {
-#pragma unroll
-                for (int k2 = 0; k2 < N2; k2++) buf[(r + N1 * k2) * ld + v] = b[k2];
-            }
-        }
-        __syncthreads();
-        // (6) split the packed real transforms, scale 1/Mx, keep modes i <= Nx/2
-        const double dn1 = 1.0 / NX;
-        for (int e = t; e < nxh * nv; e += blockDim.x) {
-            const int k = by_nv.div(e), vv = by_nv.mod(e, k);
-            const int p2 = by_rb.div(vv), r2 = by_rb.mod(vv, p2), qq = q0 + r2;
-            if (qq >= Mz) continue;
-            const double2 zk = buf[k * ld + vv];
-            const double2 zm = buf[(k == 0 ? 0 : NX - k) * ld + vv];
-            double2 A = make_double2(0.5 * (zk.x + zm.x), 0.5 * (zk.y - zm.y));
-            double2 B = make_double2(0.5 * (zk.y + zm.y), 0.5 * (zm.x - zk.x));
-            if (k == 0) {
-                A.y = 0.0;
-                B.y = 0.0;
-            }
-            S[((size_t)(2 * p2) * Mz + qq) * nxh + k] = make_double2(dn1 * A.x, dn1 * A.y);
-            S[((size_t)(2 * p2 + 1) * Mz + qq) * nxh + k] = make_double2(dn1 * B.x, dn1 * B.y);
-        }
+    constexpr int H = N1 / 2;
+    if (N2 <= N1) {
+        m = r < N2 ? r : -1;
+        partner = r < N2 ? (N2 - r) % N2 : r;
+    } else if (g == 0) {
+        m = r < H ? r : (r > H ? N2 - (N1 - r) : (N2 % 2 ? -1 : N2 / 2));
+        partner = (N1 - r) % N1;
+    } else {
+        partner = N1 - 1 - r;
+        const int a = H * g + (r < H ? r : partner);
+        m = 2 * a < N2 ? (r < H ? a : N2 - a) : -1;
     }
 }
 
-// ---------------------------------------------------------------------------
-// The same x stage with the threads of a vector in one warp.  Vector v of a
-// CTA is (z row v / 3, pair v % 3); its VT = max(N1, N2) threads are
-// consecutive, so the gather, both transforms and the split of a vector
-// are warp-local (__syncwarp), and only the products, which combine the
-// three pairs of a row, synchronise -- the 96 threads of a row group (2
-// rows at VT = 16, 4 at VT = 8) on a named barrier of their own, so the
-// groups of a CTA never wait on one another.  Each vector owns one region
-// of max(NX, N1 (N2 + 1)) complex: natural order for the gather, the
-// products and the first pass's reads, an N1 x (N2 + 1) padded matrix for
-// the exchange between the passes (conflict-free column reads).  The CFL
-// maxima are reduced per warp.  Same arithmetic as k_xprod_f, element for
-// element.
-//
-// DIRECT = 1: the first pass reads its N1 elements of the packed vector
-// straight from the staging rows in global memory (each mode's two rows are
-// read by the two lanes holding z[k] and z[NX - k]), so the gather's shared
-// memory round trip and its __syncwarp disappear.
-template <int NX, int DIRECT>
-__global__ void __launch_bounds__(LH_XPROD_T, LH_XPROD_B) k_xprod_w(const Inst *__restrict__ insts, const Work *__restrict__ work,
-                                                          int count, int rb, int want_max)
+template <int NX>
+__global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 9 ? 4 : (XPlan<NX>::N2 <= 18 ? 3 : 2))
+    k_xprod_r(const Inst *__restrict__ insts, const Work *__restrict__ work, int rb, int want_max)
 {
-    constexpr int N1 = Plan2<NX>::N1, N2 = Plan2<NX>::N2;
-    constexpr int VT = N1 > N2 ? N1 : N2;
-    if constexpr (32 % VT != 0) return;  // never launched (xprod_warp_size)
-    constexpr int LD = N2 + 1;
-    constexpr int REG = (NX > N1 * LD ? NX : N1 * LD);
-    constexpr int RG = 32 / VT;  // rows per 96-thread group
-    constexpr int nxh = NX / 3 + 1;
+    using XP = XPlan<NX>;
+    constexpr int N1 = XP::N1, N2 = XP::N2, LD = XP::LD, KQ = XP::KQ, nxh = NX / 3 + 1;
     extern __shared__ double2 sm[];
-    if ((int)blockIdx.x >= count) return;
-    const double2 *tw = insts[work[blockIdx.x].inst].twx;
-    const int t = threadIdx.x, v = t / VT, r = t % VT;
-    const int row = v / 3, pair = v % 3, grp = row / RG;
-    const double2 twr = __ldg(tw + (r < N2 ? r : 0));
     const Work w = work[blockIdx.x];
     const Inst &I = insts[w.inst];
+    const double2 *tw = I.twx;
+    const int t = threadIdx.x, lane = t & 31, r = t % N1, row = t / N1, group = lane - r;
     const int Mz = I.Mz, j = w.j;
-    const int q = w.blk * rb + row;  // this vector's z row
-    const bool live = row < rb;      // threads past the CTA's rows only join the barriers
-    const bool rowok = live && q < Mz;
-    double2 *z = sm + (size_t)(live ? v : 0) * REG;
+    const int q = w.blk * rb + row;  // this lane's z row
+    const bool rowok = row < rb && q < Mz;
+    double2 *T = sm + (size_t)row * N1 * LD;
     const size_t fs = (size_t)Mz * nxh;
-    // (0) this vector's two real rows with the y interpolations (interp_v
-    // FOU3D.f90:407, interp_u :387) as the packed Hermitian-extended complex
-    // vector z = A + iB: z[0] = (A0.x, B0.x), z[k] = A_k + iB_k and
-    // z[NX - k] = conj(A_k) + i conj(B_k) for 0 < k <= Nx/2, zero between
-    const double2 *u1j = sin_field(I, w.aux + 1, 0), *u3j = u1j + fs, *vj = u3j + fs;
-    const double2 *vjm = sin_field(I, w.aux, 2);
-    const double2 *u1p = sin_field(I, w.aux + 2, 0), *u3p = u1p + fs;
+    // this row in the planes the y interpolations (interp_v FOU3D.f90:407,
+    // interp_u :387) read
+    const size_t orow = (size_t)min(q, Mz - 1) * nxh;
+    const double2 *u1j = sin_field(I, w.aux + 1, 0) + orow, *u3j = u1j + fs, *vj = u3j + fs;
+    const double2 *vjm = sin_field(I, w.aux, 2) + orow;
+    const double2 *u1p = sin_field(I, w.aux + 2, 0) + orow, *u3p = u1p + fs;
+    double2 *S = sprod_slot(I, w.slot) + (size_t)q * nxh;
     const double dnv = 1.0 / (I.yv[j] - I.yv[j - 1]), dnu = 1.0 / (I.yu[j + 1] - I.yu[j]);
     const double w0v = (I.yu[j] - I.yv[j - 1]) * dnv, w1v = (I.yv[j] - I.yu[j]) * dnv;
     const double w0u = (I.yv[j] - I.yu[j]) * dnu, w1u = (I.yu[j + 1] - I.yv[j]) * dnu;
-    auto rows_at = [&](int k, double2 &A, double2 &B) {
-        const size_t o = (size_t)q * nxh + k;
-        if (pair == 0) {
-            A = u1j[o];
-            B = u3j[o];
-        } else if (pair == 1) {
-            const double2 x0 = vj[o], x1 = vjm[o];
-            A = make_double2(w0v * x0.x + w1v * x1.x, w0v * x0.y + w1v * x1.y);
-            B = x0;
-        } else {
-            const double2 a0 = u1p[o], a1 = u1j[o], b0 = u3p[o], b1 = u3j[o];
-            A = make_double2(w0u * a0.x + w1u * a1.x, w0u * a0.y + w1u * a1.y);
-            B = make_double2(w0u * b0.x + w1u * b1.x, w0u * b0.y + w1u * b1.y);
-        }
-    };
-    if (!DIRECT && live) {
-        constexpr int kGatherUnroll = LH_XGATHER_UNROLL;
-#pragma unroll kGatherUnroll
-        for (int k = r; k < nxh; k += VT) {
-            double2 A = make_double2(0.0, 0.0), B = A;
-            if (rowok) rows_at(k, A, B);
-            if (k == 0) {
-                z[0] = make_double2(A.x, B.x);
-            } else {
-                z[k] = make_double2(A.x - B.y, A.y + B.x);
-                z[NX - k] = make_double2(A.x + B.y, B.x - A.y);
-            }
-        }
-        for (int x = nxh + r; x <= NX - nxh; x += VT) z[x] = make_double2(0.0, 0.0);
-    }
-    if (!DIRECT) __syncwarp();
-    // (1) inverse pass 1: lane r < N2 holds n = r + N2 n1; out to the padded matrix
-    {
-        double2 a[N1];
-        if (live && r < N2) {
-            if (DIRECT) {
-#pragma unroll
-                for (int n1 = 0; n1 < N1; n1++) {
-                    const int n = r + N2 * n1;
-                    double2 A = make_double2(0.0, 0.0), B = A, y = A;
-                    if (rowok && n < nxh) {
-                        rows_at(n, A, B);
-                        y = n == 0 ? make_double2(A.x, B.x) : make_double2(A.x - B.y, A.y + B.x);
-                    } else if (rowok && n > NX - nxh) {
-                        rows_at(NX - n, A, B);
-                        y = make_double2(A.x + B.y, B.x - A.y);
-                    }
-                    a[n1] = y;
-                }
-            } else {
-#pragma unroll
-                for (int n1 = 0; n1 < N1; n1++) a[n1] = z[r + N2 * n1];
-            }
-        }
-        if (!DIRECT) __syncwarp();
-        if (live && r < N2) {
-            DFT<N1, +1, NX>::run(a, tw);
-            TwStep ts(twr);
-#pragma unroll
-            for (int k1 = 0; k1 < N1; k1++) {
-                double2 y = a[k1];
-                if (k1 > 0) y = twiddle<+1>(ts.next(), y);
-                z[k1 * LD + r] = y;
-            }
-        }
-    }
-    __syncwarp();
-    // (2) inverse pass 2 -> physical values z[x], natural order
-    {
-        double2 b[N2];
-        if (live && r < N1) {
-#pragma unroll
-            for (int n2 = 0; n2 < N2; n2++) b[n2] = z[r * LD + n2];
-            DFT<N2, +1, NX>::run(b, tw);
-        }
-        __syncwarp();
-        if (live && r < N1) {
-#pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) z[r + N1 * k2] = b[k2];
-        }
-    }
-    // (3) products of each row group's rows (the three pairs of a row sit in
-    // up to two warps of the group); CFL maxima over planes 1..nyu-1
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(96) : "memory");
     const bool track = want_max && I.dt_mode == 0 && j <= I.nyu - 1;
     double m1 = 0.0, m3 = 0.0;
-    {
-        const int gt = t - grp * 96;  // thread within the group
-        const int row0 = grp * RG;
-        for (int e = gt; e < RG * NX; e += 96) {
-            const int rr = row0 + e / NX, x = e % NX;
-            if (rr >= rb) continue;
-            double2 *p0 = sm + (size_t)(3 * rr) * REG + x, *p1 = p0 + REG, *p2 = p1 + REG;
-            const double2 a0 = *p0, a1 = *p1, a2 = *p2;
-            const double u1 = a0.x, u3 = a0.y, u2c = a1.x, u2 = a1.y, u1f = a2.x, u3f = a2.y;
-            if (track && w.blk * rb + rr < Mz) {
-                m1 = fmax(m1, fabs(u1));
-                m3 = fmax(m3, fabs(u3));
-            }
-            *p0 = make_double2(u1 * u1, u1 * u3);
-            *p1 = make_double2(u2c * u2c, u3 * u3);
-            *p2 = make_double2(u1f * u2, u3f * u2);
-        }
-    }
-    if (track) {
-        for (int o = 16; o > 0; o >>= 1) {
-            m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-            m3 = fmax(m3, __shfl_xor_sync(0xffffffffu, m3, o));
-        }
-        if ((t & 31) == 0) {
-            atomicMax(reinterpret_cast<unsigned long long *>(&I.sc[SC_U1MAX]), (unsigned long long)__double_as_longlong(m1));
-            atomicMax(reinterpret_cast<unsigned long long *>(&I.sc[SC_U3MAX]), (unsigned long long)__double_as_longlong(m3));
-        }
-    }
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(96) : "memory");
-    // (4) forward pass 1
-    {
-        double2 a[N1];
-        if (live && r < N2) {
+    double saved[N2];
+#pragma unroll 1
+    for (int pair = 0; pair < 3; pair++) {
+        // gather and inverse pass 1
+#pragma unroll 1
+        for (int g = 0; g < XP::ROUNDS; g++) {
+            int n2, partner;
+            xtask<N1, N2>(g, r, n2, partner);
+            double2 a[N1], mir[KQ], A[KQ], B[KQ];
+            // every load of the task before the first use (indices past the
+            // modes or the rows are clamped, their values dropped)
+            auto at = [&](int n1) {
+                const int k = (n2 >= 0 ? n2 : 0) + N2 * n1;
+                return k < nxh ? k : 0;
+            };
+            if (pair == 0) {  // (u1, u3) at the centre
 #pragma unroll
-            for (int n1 = 0; n1 < N1; n1++) a[n1] = z[r + N2 * n1];
-            DFT<N1, -1, NX>::run(a, tw);
-        }
-        __syncwarp();
-        if (live && r < N2) {
-            TwStep ts(twr);
-#pragma unroll
-            for (int k1 = 0; k1 < N1; k1++) {
-                double2 y = a[k1];
-                if (k1 > 0) y = twiddle<-1>(ts.next(), y);
-                z[k1 * LD + r] = y;
-            }
-        }
-    }
-    __syncwarp();
-    // (5) forward pass 2 -> X[k], natural order
-    {
-        double2 b[N2];
-        if (live && r < N1) {
-#pragma unroll
-            for (int n2 = 0; n2 < N2; n2++) b[n2] = z[r * LD + n2];
-            DFT<N2, -1, NX>::run(b, tw);
-        }
-        __syncwarp();
-        if (live && r < N1) {
-#pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) z[r + N1 * k2] = b[k2];
-        }
-    }
-    __syncwarp();
-    // (6) split the packed real transforms, scale 1/Mx, keep modes i <= Nx/2
-    if (rowok) {
-        double2 *S = sprod_slot(I, w.slot);
-        const double dn1 = 1.0 / NX;
-        for (int k = r; k < nxh; k += VT) {
-            const double2 zk = z[k];
-            const double2 zm = z[k == 0 ? 0 : NX - k];
-            double2 A = make_double2(0.5 * (zk.x + zm.x), 0.5 * (zk.y - zm.y));
-            double2 B = make_double2(0.5 * (zk.y + zm.y), 0.5 * (zm.x - zk.x));
-            if (k == 0) {
-                A.y = 0.0;
-                B.y = 0.0;
-            }
-            S[((size_t)(2 * pair) * Mz + q) * nxh + k] = make_double2(dn1 * A.x, dn1 * A.y);
-            S[((size_t)(2 * pair + 1) * Mz + q) * nxh + k] = make_double2(dn1 * B.x, dn1 * B.y);
-        }
-    }
-}
-
-// Two-pass transform of one packed vector of length NX held by the VT lanes
-// of a warp in its shared-memory region z (natural order in and out; the
-// N1 x (N2 + 1) padded matrix in between).  SGN = +1 inverse, -1 forward.
-// Every lane of the warp calls it (act = false only joins the __syncwarp).
-template <int NX, int SGN>
-__device__ __forceinline__ void xvec_fft(double2 *z, const double2 *tw, double2 twr, int r, bool act)
-{
-    constexpr int N1 = Plan2<NX>::N1, N2 = Plan2<NX>::N2;
-    constexpr int LD = N2 + 1;
-    __syncwarp();
-    {
-        double2 a[N1];
-        if (act && r < N2) {
-#pragma unroll
-            for (int n1 = 0; n1 < N1; n1++) a[n1] = z[r + N2 * n1];
-        }
-        __syncwarp();
-        if (act && r < N2) {
-            DFT<N1, SGN, NX>::run(a, tw);
-            TwStep ts(twr);
-#pragma unroll
-            for (int k1 = 0; k1 < N1; k1++) {
-                double2 y = a[k1];
-                if (k1 > 0) y = twiddle<SGN>(ts.next(), y);
-                z[k1 * LD + r] = y;
-            }
-        }
-    }
-    __syncwarp();
-    {
-        double2 b[N2];
-        if (act && r < N1) {
-#pragma unroll
-            for (int n2 = 0; n2 < N2; n2++) b[n2] = z[r * LD + n2];
-            DFT<N2, SGN, NX>::run(b, tw);
-        }
-        __syncwarp();
-        if (act && r < N1) {
-#pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) z[r + N1 * k2] = b[k2];
-        }
-    }
-    __syncwarp();
-}
-
-// ---------------------------------------------------------------------------
-// The x stage over a group of consecutive planes (the default where a
-// vector fits a warp).  The y interpolations are linear and commute with
-// the x transform too, so this stage transforms each y row's fields once --
-// (u1, u3) of a u plane as one packed vector, two adjacent v rows as
-// another -- and interpolates the physical rows of neighbouring planes: u2
-// at the u plane (interp_v, FOU3D.f90:407), u1 and u3 at the v plane
-// (interp_u, :387), with the weights of k_xprod_w.  Per plane that is 1.5
-// inverse transforms instead of 3, and 3 staging rows read instead of 8.
-//
-// A work item is a group of np <= kXGroup planes j .. j+np-1 and a block of
-// rb z rows; the plan starts groups at absolute planes 1 + kXGroup g, and v
-// rows are paired from the group's first plane, V_m = (v(j-1+2m), v(j+2m)),
-// so every row is transformed with the same partner -- and every plane's
-// products come out of the same operations -- whatever the plan's rounds,
-// staging budget or batch, as long as a round holds at least kXGroup planes
-// (below that the groups are cut at the round boundaries).  A row's physical
-// values depend on the partner packed with it at the rounding level.
-//
-// Each z row runs sub-rounds of three vectors on its three vector slots
-// (VT lanes each, one warp-local transform per vector): sub-round 0
-// transforms A_0 = (u1, u3)(j), A_1 and V_0, after which plane j's products
-// are formed and transformed forward; sub-round k >= 1 transforms A_2k,
-// A_2k+1 and V_k, after which planes j+2k-1 and j+2k follow.  Regions per z
-// row: three for the A vectors (index mod 3), two for the V vectors (mod 2)
-// and two for the second and third product pairs; the first pair (u1 u1,
-// u1 u3) overwrites A_p in place.  Row groups of 96 threads synchronise on a
-// named barrier of their own before each sub-round and around each plane's
-// products.  Same transforms, products, split and CFL maxima as k_xprod_w.
-template <int NX>
-__global__ void __launch_bounds__(LH_XMULTI_T, LH_XMULTI_B) k_xprod_m(const Inst *__restrict__ insts,
-                                                                      const Work *__restrict__ work, int count,
-                                                                      int rb, int want_max)
-{
-    constexpr int N1 = Plan2<NX>::N1, N2 = Plan2<NX>::N2;
-    constexpr int VT = N1 > N2 ? N1 : N2;
-    if constexpr (32 % VT != 0) return;  // never launched (xprod_warp_size)
-    constexpr int LD = N2 + 1;
-    constexpr int REG = (NX > N1 * LD ? NX : N1 * LD);
-    constexpr int RG = 32 / VT;  // rows per 96-thread group
-    constexpr int nxh = NX / 3 + 1;
-    constexpr int kRegions = 7;
-    extern __shared__ double2 sm[];
-    if ((int)blockIdx.x >= count) return;
-    const double2 *tw = insts[work[blockIdx.x].inst].twx;
-    const int t = threadIdx.x, v = t / VT, r = t % VT;
-    const int row = v / 3, slot = v % 3, grp = row / RG;
-    const double2 twr = __ldg(tw + (r < N2 ? r : 0));
-    const Work w = work[blockIdx.x];
-    const Inst &I = insts[w.inst];
-    const int Mz = I.Mz, j = w.j, np = w.blk >> 16;
-    const int q = (w.blk & 0xffff) * rb + row;  // this thread's z row
-    const bool live = row < rb;                  // threads past the CTA's rows only join the barriers
-    const bool rowok = live && q < Mz;
-    double2 *const R = sm + (size_t)(live ? row : 0) * kRegions * REG;
-    const size_t fs = (size_t)Mz * nxh, orow = (size_t)q * nxh;
-    const bool track = want_max && I.dt_mode == 0;
-    double m1 = 0.0, m3 = 0.0;
-    // sub-round k: the inverse transforms of A_2k, A_2k+1 and V_k
-    auto subround = [&](const int k) {
-        // the regions this sub-round fills were last read by other slots
-        if (k > 0) asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(96) : "memory");
-        double2 *z;
-        const double2 *sa = nullptr, *sb = nullptr;
-        bool act = live;
-        if (slot < 2) {
-            const int tt = 2 * k + slot;  // A_tt: (u1, u3) of plane j + tt
-            z = R + (tt % 3) * REG;
-            act = act && tt <= np;
-            sa = sin_field(I, w.aux + 1 + tt, 0);
-            sb = sa + fs;
-        } else {
-            // V_k: v rows j-1+2k and j+2k; the second is past the group only
-            // when np is even, i.e. in the last group below the top wall,
-            // where it is the ghost row above v(nyu): zero
-            z = R + (3 + (k & 1)) * REG;
-            sa = sin_field(I, w.aux + 2 * k, 2);
-            sb = 2 * k < np ? sin_field(I, w.aux + 2 * k + 1, 2) : nullptr;
-        }
-        if (act) {
-            for (int m = r; m < nxh; m += VT) {
-                double2 A = make_double2(0.0, 0.0), B = A;
-                if (rowok) {
-                    A = sa[orow + m];
-                    if (sb) B = sb[orow + m];
+                for (int n1 = 0; n1 < KQ; n1++) {
+                    A[n1] = u1j[at(n1)];
+                    B[n1] = u3j[at(n1)];
                 }
-                if (m == 0) {
-                    z[0] = make_double2(A.x, B.x);
-                } else {
-                    z[m] = make_double2(A.x - B.y, A.y + B.x);
-                    z[NX - m] = make_double2(A.x + B.y, B.x - A.y);
+            } else if (pair == 1) {  // u2 at the centre and at the face
+#pragma unroll
+                for (int n1 = 0; n1 < KQ; n1++) {
+                    A[n1] = vjm[at(n1)];
+                    B[n1] = vj[at(n1)];
+                }
+#pragma unroll
+                for (int n1 = 0; n1 < KQ; n1++)
+                    A[n1] = make_double2(w0v * B[n1].x + w1v * A[n1].x, w0v * B[n1].y + w1v * A[n1].y);
+            } else {  // (u1, u3) at the face
+                double2 a1[KQ], b1[KQ];
+#pragma unroll
+                for (int n1 = 0; n1 < KQ; n1++) {
+                    A[n1] = u1p[at(n1)];
+                    a1[n1] = u1j[at(n1)];
+                    B[n1] = u3p[at(n1)];
+                    b1[n1] = u3j[at(n1)];
+                }
+#pragma unroll
+                for (int n1 = 0; n1 < KQ; n1++) {
+                    A[n1] = make_double2(w0u * A[n1].x + w1u * a1[n1].x, w0u * A[n1].y + w1u * a1[n1].y);
+                    B[n1] = make_double2(w0u * B[n1].x + w1u * b1[n1].x, w0u * B[n1].y + w1u * b1[n1].y);
                 }
             }
-            for (int x = nxh + r; x <= NX - nxh; x += VT) z[x] = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int k1 = 0; k1 < N1; k1++) a[k1] = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int n1 = 0; n1 < KQ; n1++) {
+                const int k = n2 + N2 * n1;
+                const bool in = rowok && n2 >= 0 && k < nxh;
+                if (!in) A[n1] = B[n1] = make_double2(0.0, 0.0);
+                if (k == 0) A[n1].y = B[n1].y = 0.0;  // Im of mode 0 dropped (rft_buff.f:78-81)
+                a[n1] = make_double2(A[n1].x - B[n1].y, A[n1].y + B[n1].x);
+                mir[n1] = make_double2(A[n1].x + B[n1].y, B[n1].x - A[n1].y);
+            }
+#pragma unroll
+            for (int n1 = 0; n1 < KQ; n1++) {
+                const double2 z = make_double2(__shfl_sync(0xffffffffu, mir[n1].x, group + partner),
+                                               __shfl_sync(0xffffffffu, mir[n1].y, group + partner));
+                // z[NX - k] sits at N1 - 1 - n1 on the partner; task 0 is its own, one higher
+                const double2 own = n1 + 1 < KQ ? mir[n1 + 1] : make_double2(0.0, 0.0);
+                a[N1 - 1 - n1] = n2 == 0 ? own : z;
+            }
+            DFT<N1, +1, NX>::run(a, tw);
+            if (n2 >= 0) {
+                TwStep ts(__ldg(tw + n2));
+#pragma unroll
+                for (int k1 = 0; k1 < N1; k1++) T[k1 * LD + n2] = k1 > 0 ? twiddle<+1>(ts.next(), a[k1]) : a[k1];
+            }
         }
-        xvec_fft<NX, +1>(z, tw, twr, r, act);
-    };
-    // plane j + p: products, forward transforms and split
-    auto plane = [&](const int p) {
-        const int jp = j + p;
-        const double dnv = 1.0 / (I.yv[jp] - I.yv[jp - 1]), dnu = 1.0 / (I.yu[jp + 1] - I.yu[jp]);
-        const double w0v = (I.yu[jp] - I.yv[jp - 1]) * dnv, w1v = (I.yv[jp] - I.yu[jp]) * dnv;
-        const double w0u = (I.yv[jp] - I.yu[jp]) * dnu, w1u = (I.yu[jp + 1] - I.yv[jp]) * dnu;
-        const bool trk = track && jp <= I.nyu - 1;
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(96) : "memory");
+        __syncwarp();
+        // inverse pass 2, products, forward pass 1 of lane r's row of the matrix
         {
-            const int gt = t - grp * 96, row0 = grp * RG;
-            const int ra = p % 3, rn = (p + 1) % 3, rvm = 3 + ((p >> 1) & 1), rvv = 3 + (((p + 1) >> 1) & 1);
-            for (int e = gt; e < RG * NX; e += 96) {
-                const int rr = row0 + e / NX, x = e % NX;
-                if (rr >= rb) continue;
-                double2 *Rr = sm + (size_t)rr * kRegions * REG;
-                const double2 a0 = Rr[ra * REG + x], a1 = Rr[rn * REG + x];
-                const double2 c0 = Rr[rvm * REG + x], c1 = Rr[rvv * REG + x];
-                const double u1 = a0.x, u3 = a0.y;
-                const double vm = (p & 1) ? c0.y : c0.x;        // v(jp - 1)
-                const double u2 = ((p + 1) & 1) ? c1.y : c1.x;  // v(jp)
-                const double u2c = w0v * u2 + w1v * vm;
-                const double u1f = w0u * a1.x + w1u * u1, u3f = w0u * a1.y + w1u * u3;
-                if (trk && (w.blk & 0xffff) * rb + rr < Mz) {
-                    m1 = fmax(m1, fabs(u1));
-                    m3 = fmax(m3, fabs(u3));
+            double2 b[N2];
+#pragma unroll
+            for (int n2 = 0; n2 < N2; n2++) b[n2] = T[r * LD + n2];
+            DFT<N2, +1, NX>::run(b, tw);
+            if (pair == 0) {
+#pragma unroll
+                for (int x = 0; x < N2; x++) {
+                    const double u1 = b[x].x, u3 = b[x].y;
+                    if (track) {
+                        m1 = fmax(m1, fabs(u1));
+                        m3 = fmax(m3, fabs(u3));
+                    }
+                    saved[x] = u3 * u3;
+                    b[x] = make_double2(u1 * u1, u1 * u3);
                 }
-                Rr[ra * REG + x] = make_double2(u1 * u1, u1 * u3);
-                Rr[5 * REG + x] = make_double2(u2c * u2c, u3 * u3);
-                Rr[6 * REG + x] = make_double2(u1f * u2, u3f * u2);
+            } else if (pair == 1) {
+#pragma unroll
+                for (int x = 0; x < N2; x++) {
+                    const double u2c = b[x].x, u2 = b[x].y;
+                    b[x] = make_double2(u2c * u2c, saved[x]);
+                    saved[x] = u2;
+                }
+            } else {
+#pragma unroll
+                for (int x = 0; x < N2; x++) b[x] = make_double2(b[x].x * saved[x], b[x].y * saved[x]);
+            }
+            DFT<N2, -1, NX>::run(b, tw);
+            TwStep ts(__ldg(tw + r));
+#pragma unroll
+            for (int m = 0; m < N2; m++) T[r * LD + m] = m > 0 ? twiddle<-1>(ts.next(), b[m]) : b[m];
+        }
+        __syncwarp();
+        // forward pass 2, split, scale 1/Mx
+#pragma unroll 1
+        for (int g = 0; g < XP::ROUNDS; g++) {
+            int m, partner;
+            xtask<N1, N2>(g, r, m, partner);
+            double2 e[N1];
+#pragma unroll
+            for (int k1 = 0; k1 < N1; k1++) e[k1] = T[k1 * LD + (m >= 0 ? m : 0)];
+            DFT<N1, -1, NX>::run(e, tw);
+            const double h = 0.5 / NX;
+#pragma unroll
+            for (int k1 = 0; k1 < KQ; k1++) {
+                const double2 z = make_double2(__shfl_sync(0xffffffffu, e[N1 - 1 - k1].x, group + partner),
+                                               __shfl_sync(0xffffffffu, e[N1 - 1 - k1].y, group + partner));
+                const int k = m + N2 * k1;
+                const double2 zk = e[k1], own = e[(N1 - k1) % N1], zm = m == 0 ? own : z;
+                if (rowok && m >= 0 && k < nxh) {
+                    double2 A = make_double2(h * (zk.x + zm.x), h * (zk.y - zm.y));
+                    double2 B = make_double2(h * (zk.y + zm.y), h * (zm.x - zk.x));
+                    if (k == 0) A.y = B.y = 0.0;
+                    S[(size_t)(2 * pair) * fs + k] = A;
+                    S[(size_t)(2 * pair + 1) * fs + k] = B;
+                }
             }
         }
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(96) : "memory");
-        double2 *zf = R + (slot == 0 ? p % 3 : 4 + slot) * REG;
-        xvec_fft<NX, -1>(zf, tw, twr, r, live);
-        // split the packed real transforms, scale 1/Mx, keep modes i <= Nx/2
-        if (rowok) {
-            double2 *S = sprod_slot(I, w.slot + p);
-            const double dn1 = 1.0 / NX;
-            for (int m = r; m < nxh; m += VT) {
-                const double2 zk = zf[m];
-                const double2 zm = zf[m == 0 ? 0 : NX - m];
-                double2 A = make_double2(0.5 * (zk.x + zm.x), 0.5 * (zk.y - zm.y));
-                double2 B = make_double2(0.5 * (zk.y + zm.y), 0.5 * (zm.x - zk.x));
-                if (m == 0) {
-                    A.y = 0.0;
-                    B.y = 0.0;
-                }
-                S[((size_t)(2 * slot) * Mz + q) * nxh + m] = make_double2(dn1 * A.x, dn1 * A.y);
-                S[((size_t)(2 * slot + 1) * Mz + q) * nxh + m] = make_double2(dn1 * B.x, dn1 * B.y);
-            }
-        }
-    };
-    // straight-line code for the group size: as a runtime loop over the
-    // sub-rounds the compiler keeps values live across iterations and spills
-    // (168 registers and 1.3 KB of spills at Mx = 192, against 124 and none)
-    static_assert(kXGroup == 5, "the sequence below covers groups of five planes");
-    subround(0);
-    plane(0);
-    if (np > 1) {
-        subround(1);
-        plane(1);
-        if (np > 2) plane(2);
     }
-    if (np > 3) {
-        subround(2);
-        plane(3);
-        if (np > 4) plane(4);
-    }
-    if (track) {
+    if (track) {  // CFL maxima over planes 1..nyu-1; rows past the last are zero
         for (int o = 16; o > 0; o >>= 1) {
             m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
             m3 = fmax(m3, __shfl_xor_sync(0xffffffffu, m3, o));
         }
-        if ((t & 31) == 0) {
+        if (lane == 0) {
             atomicMax(reinterpret_cast<unsigned long long *>(&I.sc[SC_U1MAX]), (unsigned long long)__double_as_longlong(m1));
             atomicMax(reinterpret_cast<unsigned long long *>(&I.sc[SC_U3MAX]), (unsigned long long)__double_as_longlong(m3));
         }
@@ -1050,8 +631,7 @@ __global__ void __launch_bounds__(LH_ZFWD_T, LH_ZFWD_B) k_zfwd_w(const Inst *__r
 
 // ---------------------------------------------------------------------------
 // host dispatch
-int fast_max_threads(int stage) { return stage == 0 ? LH_ZINV_T : (stage == 1 ? LH_XPROD_T : LH_ZFWD_T); }
-int xprod_max_threads(int n) { return xprod_multi(n) ? LH_XMULTI_T : LH_XPROD_T; }
+int fast_max_threads(int stage) { return stage == 0 ? LH_ZINV_T : LH_ZFWD_T; }
 
 bool fast_size(int n)
 {
@@ -1099,7 +679,7 @@ int fast_threads(int n, int vectors)
 
 // z-inverse sizes whose vectors fit a warp (max(N1, N2) divides 32), and
 // whether the warp-local variant is selected (LH_ZINV_WARP=1).
-bool zinv_warp_size(int n)
+static bool zinv_warp_size(int n)
 {
     switch (n) {
 #define LH_CASE(N) \
@@ -1112,61 +692,50 @@ bool zinv_warp_size(int n)
     }
 }
 
-bool zinv_warp(int n)
+static bool zinv_warp(int n)
 {
     const char *ev = getenv("LH_ZINV_WARP");
     return ev && ev[0] == '1' && zinv_warp_size(n);
 }
 
-// x stage: sizes whose vectors fit a warp, and the variant selection.
-// Where a vector fits a warp the warp-local k_xprod_w is the default
-// (measured on B200 at 128x128x153: x products 0.256 -> 0.236 ms per
-// substep, step 1.283 -> 1.218 ms); LH_XPROD_WARP selects the others for
-// measurement: 0 the block-synchronous k_xprod_f, 2 k_xprod_w's direct-read
-// form, 3 the multi-plane k_xprod_m.
-bool xprod_warp_size(int n) { return zinv_warp_size(n); }
-static int xprod_mode(int n)
+// x stage: z rows per CTA for a bound rb (whole warps, at most kXprodThreads
+// lanes), its threads and shared memory
+int xprod_rows(int n, int rb)
 {
-    if (!xprod_warp_size(n)) return 0;
-    const char *ev = getenv("LH_XPROD_WARP");
-    if (!ev || !*ev || ev[0] == '1') return 1;
-    return ev[0] == '3' ? 3 : (ev[0] == '2' ? 2 : 0);
+    switch (n) {
+#define LH_CASE(N) \
+    case N: return XPlan<N>::RW * std::max(1, std::min(kXprodThreads / 32, (rb + XPlan<N>::RW - 1) / XPlan<N>::RW));
+        LH_FAST_SIZES(LH_CASE)
+#undef LH_CASE
+    default: return 1;
+    }
 }
-bool xprod_warp(int n) { return xprod_mode(n) != 0; }
-bool xprod_multi(int n) { return xprod_mode(n) == 3; }
 
-// Threads and shared memory of an x-stage CTA of rb z rows: the warp variants
-// run 96-thread row groups (32 / VT rows each), one region per vector
-// (k_xprod_w) or seven per z row (k_xprod_m).
 int xprod_threads(int n, int rb)
 {
-    if (!xprod_warp(n)) return fast_threads(n, 3 * rb);
-    const int vt = fast_vector_threads(n), rg = 32 / vt;
-    return 96 * ((rb + rg - 1) / rg);
+    switch (n) {
+#define LH_CASE(N) \
+    case N: return rb / XPlan<N>::RW * 32;
+        LH_FAST_SIZES(LH_CASE)
+#undef LH_CASE
+    default: return 0;
+    }
 }
 
 size_t xprod_smem(int n, int rb)
 {
-    const int mode = xprod_mode(n);
-    if (mode == 0) return (size_t)n * ((3 * rb) | 1) * sizeof(double2);
-    const int per_row = mode == 3 ? 7 : 3;
     switch (n) {
-#define LH_CASE(N)                                                                                  \
-    case N: {                                                                                       \
-        const int reg = N > Plan2<N>::N1 * (Plan2<N>::N2 + 1) ? N : Plan2<N>::N1 * (Plan2<N>::N2 + 1); \
-        const int rg = 32 / fast_vector_threads(N);                                                 \
-        return (size_t)per_row * rg * ((rb + rg - 1) / rg) * reg * sizeof(double2);               \
-    }
+#define LH_CASE(N) \
+    case N: return (size_t)rb * XPlan<N>::N1 * XPlan<N>::LD * sizeof(double2);
         LH_FAST_SIZES(LH_CASE)
 #undef LH_CASE
-    default:
-        return 0;
+    default: return 0;
     }
 }
 
 // z forward: sizes whose vectors fit a warp, the LH_ZFWD_WARP=1 selection,
 // threads and shared memory of a CTA of cb x modes (3 cb vectors)
-bool zfwd_warp(int n)
+static bool zfwd_warp(int n)
 {
     const char *ev = getenv("LH_ZFWD_WARP");
     return ev && ev[0] == '1' && zinv_warp_size(n);
@@ -1229,10 +798,7 @@ cudaError_t fast_set_attributes(int Mz, int Mx, size_t smz, size_t smx, size_t s
     switch (Mx) {
 #define LH_CASE(N)                                         \
     case N:                                                \
-        e = raise_smem_limit((const void *)k_xprod_f<N>, smx); \
-        if (e == cudaSuccess) e = raise_smem_limit((const void *)k_xprod_w<N, 0>, smx); \
-        if (e == cudaSuccess) e = raise_smem_limit((const void *)k_xprod_w<N, 1>, smx); \
-        if (e == cudaSuccess) e = raise_smem_limit((const void *)k_xprod_m<N>, smx); \
+        e = raise_smem_limit((const void *)k_xprod_r<N>, smx); \
         break;
         LH_FAST_SIZES(LH_CASE)
 #undef LH_CASE
@@ -1262,12 +828,7 @@ void fast_launch_xprod(int Mx, unsigned grid, int threads, size_t smem, cudaStre
     switch (Mx) {
 #define LH_CASE(N)                                                                   \
     case N:                                                                          \
-        switch (xprod_mode(N)) {                                                     \
-        case 3: k_xprod_m<N><<<grid, threads, smem, st>>>(insts, work, count, rb, want_max); break; \
-        case 2: k_xprod_w<N, 1><<<grid, threads, smem, st>>>(insts, work, count, rb, want_max); break; \
-        case 1: k_xprod_w<N, 0><<<grid, threads, smem, st>>>(insts, work, count, rb, want_max); break; \
-        default: k_xprod_f<N><<<grid, threads, smem, st>>>(insts, work, count, rb, want_max); \
-        }                                                                            \
+        k_xprod_r<N><<<grid, threads, smem, st>>>(insts, work, rb, want_max);        \
         break;
         LH_FAST_SIZES(LH_CASE)
 #undef LH_CASE
