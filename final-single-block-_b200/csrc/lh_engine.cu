@@ -311,6 +311,7 @@ static long tile_columns(int max_nyu) { return (max_nyu < 64 ? 2 : 3) * 1184L; }
 namespace {
 struct ClassTiles {
     bool fast;
+    bool small = false;  // one CTA per plane (k_plane_small): a single stage, no staging
     int cbz, rbx, cbf;
     int tz, tx, tf;
     size_t smz, smx, smf;
@@ -440,7 +441,13 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
     std::vector<const HostSetup *> rep(ncls, nullptr);
     for (size_t q = 0; q < insts.size(); q++)
         if (!rep[cls_of[q]]) rep[cls_of[q]] = &insts[q]->hs;
-    for (size_t c = 0; c < ncls; c++) tiles[c] = class_tiles(*rep[c], force_generic, force);
+    for (size_t c = 0; c < ncls; c++) {
+        tiles[c] = class_tiles(*rep[c], force_generic, force);
+        long planes = 0;
+        for (size_t q = 0; q < insts.size(); q++)
+            if (cls_of[q] == (int)c) planes += insts[q]->hs.nyu;
+        tiles[c].small = tiles[c].fast && small_plane_pays(rep[c]->Mx, rep[c]->Mz, planes);
+    }
     // staging budget and column-pass launches: the candidate, else the
     // environment, else the tuned entry of a single-class plan, else defaults
     TuneParams tuned;
@@ -467,6 +474,7 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
         // launches (16^2 x 44 24.2 -> 22.6 us a substep, x 97 28.8 -> 27.4, 32^2 x
         // 97 34.2 -> 33.5, x 153 44.6 -> 46.1)
         if (fast && insts.size() == 1 && insts[q]->inst.chunk >= s.nyu && (long)s.nc * s.nyu <= kOneRoundRows) c = s.nyu;
+        if (tiles[cls_of[q]].small) c = s.nyu;  // no staging: one round
         chunk_eff[q] = (int)c;
         rounds = std::max(rounds, (s.nyu + chunk_eff[q] - 1) / chunk_eff[q]);
     }
@@ -502,7 +510,9 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
         const int nbz = (s.nxh + ct.cbz - 1) / ct.cbz;
         const int nbx = (s.Mz + ct.rbx - 1) / ct.rbx;
         const int nbf = (s.nxh + ct.cbf - 1) / ct.cbf;
-        if (ct.fast) {
+        if (ct.small) {
+            for (int j = 1; j <= s.nyu; j++) lists[0][1][cls_of[q]].push_back({q, j, 0, 0, 0});
+        } else if (ct.fast) {
             // round r: planes j0..j1 in staging half r%2; Sin slot sb+p holds
             // y row j0-1+p (u1/u3 on rows j0..j1+1, u2 on rows j0-1..j1),
             // Sprod slot pb+j-j0 plane j
@@ -545,6 +555,7 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
                 Group g;
                 g.stage = stg;
                 g.fast = tiles[c].fast;
+                g.small = tiles[c].small;
                 g.Mz = classes[c].first;
                 g.Mx = classes[c].second;
                 g.off = all.size();
@@ -642,7 +653,9 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
     // dynamic shared-memory limits for every kernel this plan launches
     size_t gz = 0, gx = 0, gf = 0;
     for (size_t c = 0; c < ncls; c++) {
-        if (tiles[c].fast) {
+        if (tiles[c].small) {
+            if ((e = small_plane_attributes(classes[c].second, classes[c].first)) != cudaSuccess) return e;
+        } else if (tiles[c].fast) {
             if ((e = fast_set_attributes(classes[c].first, classes[c].second, tiles[c].smz, tiles[c].smx,
                                          tiles[c].smf)) != cudaSuccess)
                 return e;
@@ -756,7 +769,9 @@ cudaError_t launch_substep(const Plan &p, const Inst *d_insts, int kRK, bool cfl
             cudaStream_t st0 = st;
             cudaStream_t st = (nstreams > 1 && si > 0) ? p.side[si - 1] : st0;
             time_begin(timer, st);
-            if (g.fast) {
+            if (g.small) {
+                small_plane_launch(g.Mx, g.Mz, g.grid, st, d_insts, w, want_max);
+            } else if (g.fast) {
                 const int cnt = (int)g.count;
                 if (g.stage == 0) fast_launch_zinv(g.Mz, g.grid, g.threads, g.smem, st, d_insts, w, cnt, g.param);
                 else if (g.stage == 1)

@@ -84,6 +84,7 @@ cudaError_t omega_x_planes(const Inst *d_inst, const HostSetup &hs, const StatsS
 struct Group {
     int stage = 0;        // 0 z inverse, 1 x products, 2 z forward
     bool fast = false;    // compile-time-sized kernels
+    bool small = false;   // the whole plane pass in one kernel (stage 1 of the only round)
     int Mz = 0, Mx = 0;
     size_t off = 0, count = 0;
     int threads = 256;

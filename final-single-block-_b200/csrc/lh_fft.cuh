@@ -178,6 +178,7 @@ constexpr bool smooth23(int n)
 }
 constexpr int plan2_n1(int N)
 {
+    if (N == 24) return 8;  // 8 x 3: the z outputs kept are whole blocks of the second pass
     const int cand[8] = {16, 12, 9, 8, 6, 4, 3, 2};
     int best = 1, score = N;
     for (int k = 0; k < 8; k++) {

@@ -46,6 +46,12 @@ void launch_spectra_accumulate(const Inst *d_inst, double *sp, int nyu, int nc, 
 // raise (never lower) a kernel's dynamic shared-memory limit (lh_engine.cu)
 cudaError_t raise_smem_limit(const void *func, size_t bytes);
 
+// the plane pass of a small plane in one CTA (lh_plane_small.cu)
+bool small_plane(int Mx, int Mz);
+bool small_plane_pays(int Mx, int Mz, long planes);
+cudaError_t small_plane_attributes(int Mx, int Mz);
+void small_plane_launch(int Mx, int Mz, unsigned grid, cudaStream_t st, const Inst *insts, const Work *work, int want_max);
+
 // compile-time-sized fast path (lh_plane_fast.cu)
 bool fast_size(int n);
 int fast_threads(int n, int vectors);

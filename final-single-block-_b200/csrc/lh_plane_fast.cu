@@ -53,24 +53,11 @@
 #endif
 #define LH_MINB(N, B) ((N) >= LH_LARGE_N ? LH_LARGE_B : (B))
 #include "lh_kernels.cuh"
+#include "lh_xprod.cuh"
 
 namespace lh {
 
 constexpr int kXprodThreads = 128;  // most threads of a k_xprod_r CTA
-
-// Outer twiddles W^(r k1), k1 = 1.., of a two-pass transform by the
-// recurrence W^(r k1) = W^(r (k1-1)) W^r from one table entry, which keeps the
-// per-point table reads out of the shared-memory pipe (the kernels' busiest
-// unit); the recurrence's rounding stays within a few ulp for k1 <= 24.
-struct TwStep {
-    double2 w1, wk;
-    __device__ explicit TwStep(double2 base) : w1(base), wk(make_double2(1.0, 0.0)) {}
-    __device__ __forceinline__ double2 next()
-    {
-        wk = make_double2(wk.x * w1.x - wk.y * w1.y, wk.x * w1.y + wk.y * w1.x);
-        return wk;
-    }
-};
 
 __device__ __forceinline__ double2 *sin_field(const Inst &I, int p, int f)
 {
@@ -201,33 +188,9 @@ __global__ void __launch_bounds__(LH_ZINV_T, LH_ZINV_B) k_zinv_w(const Inst *__r
 }
 
 // ---------------------------------------------------------------------------
-// x transforms and products of one (plane j, block of z rows), the products in
-// registers.  N1 lanes of a warp own a z row and take its three vectors (pairs)
-// in turn; NX = N1 N2.
-//
-//   gather   the lane of task n2 loads the modes k = n2 + N2 q <= Nx/2 of the
-//            pair's two real rows A, B (with the y interpolations), forms z[k] =
-//            A + iB for itself and z[NX - k] = conj(A) + i conj(B) for the lane
-//            of task N2 - n2 (one shuffle), so the inputs of the inverse
-//            transform never pass through shared memory;
-//   inverse  DFT over N1, twiddle, exchange through the row's N1 x N2 matrix,
-//            DFT over N2: lane r holds the physical values x = r + N1 t;
-//   products in registers: u3^2 of the first pair waits for the second, u2 of
-//            the second for the third;
-//   forward  the mirrored split (DFT over N2 first, in the registers that hold
-//            the products), exchange, DFT over N1: the lane of task m holds the
-//            modes k = m + N2 q;
-//   split    the packed real transforms need Z[NX - k], on the lane of task
-//            N2 - m: one shuffle again; modes i <= Nx/2 are stored.
-//
-// A vector crosses shared memory twice (the exchanges, 4 accesses an element)
-// instead of 12 accesses when the gather, the products and the split went
-// through it too, which kept that pipe busier than the FP64 pipe.  Tasks come in
-// rounds of N1 whose sets are closed under m -> N2 - m, and a lane keeps its
-// columns of the matrix from one use to the next, so two __syncwarp a vector are
-// all the synchronisation.  Every load of a task is issued before the first is
-// used: loaded mode by mode the stage waited on L2 for half its time.
-//
+// x transforms and products of one (plane j, block of rb z rows): xrow on rows
+// gathered from Sin with the y interpolations (interp_v FOU3D.f90:407, interp_u
+// :387): u1(j), u3(j); u2 at centre j, u2(j); u1, u3 at face j -> Sprod[slot]
 // What bounds it: the FP64 pipe, 48 % busy (55 % on the busiest SM), at the
 // warps that 168 registers leave (three CTAs of 128); then the L2 gather and the
 // launch's last wave.  x products alone, us a substep on B200, before (one
@@ -237,206 +200,68 @@ __global__ void __launch_bounds__(LH_ZINV_T, LH_ZINV_B) k_zinv_w(const Inst *__r
 // Four CTAs an SM (128 registers) spill: 372 us at 128^2, 1764 at 192^2; three
 // instead of two at Mx = 384 3150.
 template <int NX>
-struct XPlan {
-    // the substep at the other splits, us: 192 as 8 x 24 394 (16 x 12: 362), 144 as
-    // 8 x 18 153 (148), 96 as 4 x 24 129 and 16 x 6 123 (114), 48 as 4 x 12 51 (44)
-    static constexpr int N1 = NX == 12 ? 4 : (NX <= 96 ? 8 : 16);
-    static constexpr int N2 = NX / N1;
-    static constexpr int LD = N2 | 1;             // odd row stride: conflict-free rows and columns
-    static constexpr int KQ = NX / 3 / N2 + 1;    // modes k <= Nx/2 of a task, at most
-    static constexpr int ROUNDS = N2 <= N1 ? 1 : ((N2 + 1) / 2 + N1 / 2 - 1) / (N1 / 2);
-    static constexpr int RW = 32 / N1;            // rows per warp
-};
-// Task of lane r in round g and the lane that holds task N2 - m; -1: idle.
-// Round 0: m = 0 .. N1/2 - 1, N2/2, and the mirror images N2 - m downwards from
-// the last lane; round g: m = N1/2 g + .. and its mirror images.
-template <int N1, int N2>
-__device__ __forceinline__ void xtask(int g, int r, int &m, int &partner)
-{
-    constexpr int H = N1 / 2;
-    if (N2 <= N1) {
-        m = r < N2 ? r : -1;
-        partner = r < N2 ? (N2 - r) % N2 : r;
-    } else if (g == 0) {
-        m = r < H ? r : (r > H ? N2 - (N1 - r) : (N2 % 2 ? -1 : N2 / 2));
-        partner = (N1 - r) % N1;
-    } else {
-        partner = N1 - 1 - r;
-        const int a = H * g + (r < H ? r : partner);
-        m = 2 * a < N2 ? (r < H ? a : N2 - a) : -1;
-    }
-}
-
-template <int NX>
 __global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 9 ? 4 : (XPlan<NX>::N2 <= 18 ? 3 : 2))
     k_xprod_r(const Inst *__restrict__ insts, const Work *__restrict__ work, int rb, int want_max)
 {
     using XP = XPlan<NX>;
-    constexpr int N1 = XP::N1, N2 = XP::N2, LD = XP::LD, KQ = XP::KQ, nxh = NX / 3 + 1;
+    constexpr int KQ = XP::KQ, nxh = NX / 3 + 1;
     extern __shared__ double2 sm[];
     const Work w = work[blockIdx.x];
     const Inst &I = insts[w.inst];
-    const double2 *tw = I.twx;
-    const int t = threadIdx.x, lane = t & 31, r = t % N1, row = t / N1, group = lane - r;
+    const int t = threadIdx.x, r = t % XP::N1, row = t / XP::N1;
     const int Mz = I.Mz, j = w.j;
     const int q = w.blk * rb + row;  // this lane's z row
     const bool rowok = row < rb && q < Mz;
-    double2 *T = sm + (size_t)row * N1 * LD;
-    const size_t fs = (size_t)Mz * nxh;
-    // this row in the planes the y interpolations (interp_v FOU3D.f90:407,
-    // interp_u :387) read
-    const size_t orow = (size_t)min(q, Mz - 1) * nxh;
+    // this row in the planes the y interpolations read
+    const size_t fs = (size_t)Mz * nxh, orow = (size_t)min(q, Mz - 1) * nxh;
     const double2 *u1j = sin_field(I, w.aux + 1, 0) + orow, *u3j = u1j + fs, *vj = u3j + fs;
     const double2 *vjm = sin_field(I, w.aux, 2) + orow;
     const double2 *u1p = sin_field(I, w.aux + 2, 0) + orow, *u3p = u1p + fs;
-    double2 *S = sprod_slot(I, w.slot) + (size_t)q * nxh;
+    double2 *S = sprod_slot(I, w.slot) + orow;
     const double dnv = 1.0 / (I.yv[j] - I.yv[j - 1]), dnu = 1.0 / (I.yu[j + 1] - I.yu[j]);
     const double w0v = (I.yu[j] - I.yv[j - 1]) * dnv, w1v = (I.yv[j] - I.yu[j]) * dnv;
     const double w0u = (I.yv[j] - I.yu[j]) * dnu, w1u = (I.yu[j + 1] - I.yv[j]) * dnu;
-    const bool track = want_max && I.dt_mode == 0 && j <= I.nyu - 1;
+    const bool track = want_max && I.dt_mode == 0 && j <= I.nyu - 1;  // maxima over planes 1..nyu-1
     double m1 = 0.0, m3 = 0.0;
-    double saved[N2];
-#pragma unroll 1
-    for (int pair = 0; pair < 3; pair++) {
-        // gather and inverse pass 1
-#pragma unroll 1
-        for (int g = 0; g < XP::ROUNDS; g++) {
-            int n2, partner;
-            xtask<N1, N2>(g, r, n2, partner);
-            double2 a[N1], mir[KQ], A[KQ], B[KQ];
-            // every load of the task before the first use (indices past the
-            // modes or the rows are clamped, their values dropped)
-            auto at = [&](int n1) {
-                const int k = (n2 >= 0 ? n2 : 0) + N2 * n1;
-                return k < nxh ? k : 0;
-            };
+    xrow<NX>(
+        sm + (size_t)row * XP::N1 * XP::LD, I.twx, r, rowok, track, m1, m3,
+        [&](int pair, const int *k, double2 *A, double2 *B) {
             if (pair == 0) {  // (u1, u3) at the centre
 #pragma unroll
                 for (int n1 = 0; n1 < KQ; n1++) {
-                    A[n1] = u1j[at(n1)];
-                    B[n1] = u3j[at(n1)];
+                    A[n1] = u1j[k[n1]];
+                    B[n1] = u3j[k[n1]];
                 }
             } else if (pair == 1) {  // u2 at the centre and at the face
 #pragma unroll
                 for (int n1 = 0; n1 < KQ; n1++) {
-                    A[n1] = vjm[at(n1)];
-                    B[n1] = vj[at(n1)];
+                    A[n1] = vjm[k[n1]];
+                    B[n1] = vj[k[n1]];
                 }
 #pragma unroll
                 for (int n1 = 0; n1 < KQ; n1++)
-                    A[n1] = make_double2(w0v * B[n1].x + w1v * A[n1].x, w0v * B[n1].y + w1v * A[n1].y);
+                    A[n1] = lerp(w0v, B[n1], w1v, A[n1]);
             } else {  // (u1, u3) at the face
                 double2 a1[KQ], b1[KQ];
 #pragma unroll
                 for (int n1 = 0; n1 < KQ; n1++) {
-                    A[n1] = u1p[at(n1)];
-                    a1[n1] = u1j[at(n1)];
-                    B[n1] = u3p[at(n1)];
-                    b1[n1] = u3j[at(n1)];
+                    A[n1] = u1p[k[n1]];
+                    a1[n1] = u1j[k[n1]];
+                    B[n1] = u3p[k[n1]];
+                    b1[n1] = u3j[k[n1]];
                 }
 #pragma unroll
                 for (int n1 = 0; n1 < KQ; n1++) {
-                    A[n1] = make_double2(w0u * A[n1].x + w1u * a1[n1].x, w0u * A[n1].y + w1u * a1[n1].y);
-                    B[n1] = make_double2(w0u * B[n1].x + w1u * b1[n1].x, w0u * B[n1].y + w1u * b1[n1].y);
+                    A[n1] = lerp(w0u, A[n1], w1u, a1[n1]);
+                    B[n1] = lerp(w0u, B[n1], w1u, b1[n1]);
                 }
             }
-#pragma unroll
-            for (int k1 = 0; k1 < N1; k1++) a[k1] = make_double2(0.0, 0.0);
-#pragma unroll
-            for (int n1 = 0; n1 < KQ; n1++) {
-                const int k = n2 + N2 * n1;
-                const bool in = rowok && n2 >= 0 && k < nxh;
-                if (!in) A[n1] = B[n1] = make_double2(0.0, 0.0);
-                if (k == 0) A[n1].y = B[n1].y = 0.0;  // Im of mode 0 dropped (rft_buff.f:78-81)
-                a[n1] = make_double2(A[n1].x - B[n1].y, A[n1].y + B[n1].x);
-                mir[n1] = make_double2(A[n1].x + B[n1].y, B[n1].x - A[n1].y);
-            }
-#pragma unroll
-            for (int n1 = 0; n1 < KQ; n1++) {
-                const double2 z = make_double2(__shfl_sync(0xffffffffu, mir[n1].x, group + partner),
-                                               __shfl_sync(0xffffffffu, mir[n1].y, group + partner));
-                // z[NX - k] sits at N1 - 1 - n1 on the partner; task 0 is its own, one higher
-                const double2 own = n1 + 1 < KQ ? mir[n1 + 1] : make_double2(0.0, 0.0);
-                a[N1 - 1 - n1] = n2 == 0 ? own : z;
-            }
-            DFT<N1, +1, NX>::run(a, tw);
-            if (n2 >= 0) {
-                TwStep ts(__ldg(tw + n2));
-#pragma unroll
-                for (int k1 = 0; k1 < N1; k1++) T[k1 * LD + n2] = k1 > 0 ? twiddle<+1>(ts.next(), a[k1]) : a[k1];
-            }
-        }
-        __syncwarp();
-        // inverse pass 2, products, forward pass 1 of lane r's row of the matrix
-        {
-            double2 b[N2];
-#pragma unroll
-            for (int n2 = 0; n2 < N2; n2++) b[n2] = T[r * LD + n2];
-            DFT<N2, +1, NX>::run(b, tw);
-            if (pair == 0) {
-#pragma unroll
-                for (int x = 0; x < N2; x++) {
-                    const double u1 = b[x].x, u3 = b[x].y;
-                    if (track) {
-                        m1 = fmax(m1, fabs(u1));
-                        m3 = fmax(m3, fabs(u3));
-                    }
-                    saved[x] = u3 * u3;
-                    b[x] = make_double2(u1 * u1, u1 * u3);
-                }
-            } else if (pair == 1) {
-#pragma unroll
-                for (int x = 0; x < N2; x++) {
-                    const double u2c = b[x].x, u2 = b[x].y;
-                    b[x] = make_double2(u2c * u2c, saved[x]);
-                    saved[x] = u2;
-                }
-            } else {
-#pragma unroll
-                for (int x = 0; x < N2; x++) b[x] = make_double2(b[x].x * saved[x], b[x].y * saved[x]);
-            }
-            DFT<N2, -1, NX>::run(b, tw);
-            TwStep ts(__ldg(tw + r));
-#pragma unroll
-            for (int m = 0; m < N2; m++) T[r * LD + m] = m > 0 ? twiddle<-1>(ts.next(), b[m]) : b[m];
-        }
-        __syncwarp();
-        // forward pass 2, split, scale 1/Mx
-#pragma unroll 1
-        for (int g = 0; g < XP::ROUNDS; g++) {
-            int m, partner;
-            xtask<N1, N2>(g, r, m, partner);
-            double2 e[N1];
-#pragma unroll
-            for (int k1 = 0; k1 < N1; k1++) e[k1] = T[k1 * LD + (m >= 0 ? m : 0)];
-            DFT<N1, -1, NX>::run(e, tw);
-            const double h = 0.5 / NX;
-#pragma unroll
-            for (int k1 = 0; k1 < KQ; k1++) {
-                const double2 z = make_double2(__shfl_sync(0xffffffffu, e[N1 - 1 - k1].x, group + partner),
-                                               __shfl_sync(0xffffffffu, e[N1 - 1 - k1].y, group + partner));
-                const int k = m + N2 * k1;
-                const double2 zk = e[k1], own = e[(N1 - k1) % N1], zm = m == 0 ? own : z;
-                if (rowok && m >= 0 && k < nxh) {
-                    double2 A = make_double2(h * (zk.x + zm.x), h * (zk.y - zm.y));
-                    double2 B = make_double2(h * (zk.y + zm.y), h * (zm.x - zk.x));
-                    if (k == 0) A.y = B.y = 0.0;
-                    S[(size_t)(2 * pair) * fs + k] = A;
-                    S[(size_t)(2 * pair + 1) * fs + k] = B;
-                }
-            }
-        }
-    }
-    if (track) {  // CFL maxima over planes 1..nyu-1; rows past the last are zero
-        for (int o = 16; o > 0; o >>= 1) {
-            m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-            m3 = fmax(m3, __shfl_xor_sync(0xffffffffu, m3, o));
-        }
-        if (lane == 0) {
-            atomicMax(reinterpret_cast<unsigned long long *>(&I.sc[SC_U1MAX]), (unsigned long long)__double_as_longlong(m1));
-            atomicMax(reinterpret_cast<unsigned long long *>(&I.sc[SC_U3MAX]), (unsigned long long)__double_as_longlong(m3));
-        }
-    }
+        },
+        [&](int pair, int k, double2 A, double2 B) {
+            S[(size_t)(2 * pair) * fs + k] = A;
+            S[(size_t)(2 * pair + 1) * fs + k] = B;
+        });
+    if (track) xmax(I, m1, m3);
 }
 
 // ---------------------------------------------------------------------------
@@ -511,8 +336,8 @@ __global__ void __launch_bounds__(LH_ZFWD_T, LH_MINB(NZ, LH_ZFWD_B)) k_zfwd_f(co
             if (h == 0) {  // p0 uu, p1 uw, p2 ww
                 double2 n1 = make_double2(0.0, 0.0), n3 = n1;
                 if (keep) {
-                    n1 = make_double2(-(kx * p0.y) + -(kz * p1.y), kx * p0.x + kz * p1.x);
-                    n3 = make_double2(-(kx * p1.y) + -(kz * p2.y), kx * p1.x + kz * p2.x);
+                    n1 = add_ik(kz, p1, ik(kx, p0));
+                    n3 = add_ik(kz, p2, ik(kx, p1));
                 }
                 I.NXZ1[on] = n1;
                 I.NXZ3[on] = n3;
@@ -522,7 +347,7 @@ __global__ void __launch_bounds__(LH_ZFWD_T, LH_MINB(NZ, LH_ZFWD_B)) k_zfwd_f(co
                 I.UVF[o] = p1;
                 I.WVF[o] = p2;
                 double2 n2 = make_double2(0.0, 0.0);
-                if (keep) n2 = make_double2(-(kx * p1.y) + -(kz * p2.y), kx * p1.x + kz * p2.x);
+                if (keep) n2 = add_ik(kz, p2, ik(kx, p1));
                 I.NXZ2[on] = n2;
             }
         }
@@ -612,8 +437,8 @@ __global__ void __launch_bounds__(LH_ZFWD_T, LH_ZFWD_B) k_zfwd_w(const Inst *__r
         if (h == 0) {  // p0 uu, p1 uw, p2 ww
             double2 n1 = make_double2(0.0, 0.0), n3 = n1;
             if (keep) {
-                n1 = make_double2(-(kx * p0.y) + -(kz * p1.y), kx * p0.x + kz * p1.x);
-                n3 = make_double2(-(kx * p1.y) + -(kz * p2.y), kx * p1.x + kz * p2.x);
+                n1 = add_ik(kz, p1, ik(kx, p0));
+                n3 = add_ik(kz, p2, ik(kx, p1));
             }
             I.NXZ1[on] = n1;
             I.NXZ3[on] = n3;
@@ -623,7 +448,7 @@ __global__ void __launch_bounds__(LH_ZFWD_T, LH_ZFWD_B) k_zfwd_w(const Inst *__r
             I.UVF[o] = p1;
             I.WVF[o] = p2;
             double2 n2 = make_double2(0.0, 0.0);
-            if (keep) n2 = make_double2(-(kx * p1.y) + -(kz * p2.y), kx * p1.x + kz * p2.x);
+            if (keep) n2 = add_ik(kz, p2, ik(kx, p1));
             I.NXZ2[on] = n2;
         }
     }

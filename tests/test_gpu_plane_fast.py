@@ -31,3 +31,28 @@ def test_fast_plane_pass_matches_the_generic_one(Nx, Nz, monkeypatch):
     for f in ("u1", "u2", "u3", "p"):
         assert rel_l2(out[1][0][f], out[0][0][f]) <= (1e-12 if f == "p" else 1e-13), f
     assert abs(out[1][1]["t"] - out[0][1]["t"]) <= 1e-13 * out[0][1]["t"]
+
+
+def test_one_cta_planes_are_the_staged_planes(monkeypatch):
+    """Enough planes of 48 x 48 points in a batch take the plane pass that keeps
+    a plane in one CTA; a lone instance takes the staged kernels.  The same
+    operations: the states agree bit for bit (one column pass for both)."""
+    import numpy as np
+    from lh_b200 import Batch, Desc, Engine, grids, perturbed_laminar
+    monkeypatch.setenv("LH_SMALL_COLUMNS", "0")
+    descs = [Desc(Nx=32, Nz=32, ny=ny, dt_mode=k % 2, dt=1e-3, CFL=0.5) for k, ny in enumerate((153, 153, 98))]
+    ics = [perturbed_laminar(d, 50 + k, *grids(d)) for k, d in enumerate(descs)]
+    b = Batch()
+    slots = [b.add(d, *ic) for d, ic in zip(descs, ics)]
+    b.step(2)
+    b.synchronize()
+    for d, s, ic in zip(descs, slots, ics):
+        e = Engine(d)
+        e.upload(*ic)
+        e.step(2)
+        e.synchronize()
+        want, got = e.download(), b.download(s)
+        for f in ("u1", "u2", "u3", "p"):
+            assert np.array_equal(got[f], want[f]), f
+        e.close()
+    b.close()
