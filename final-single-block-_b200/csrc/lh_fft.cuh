@@ -168,8 +168,8 @@ struct DFT<4, SGN, NT> {
 
 // Two-pass split N = N1 * N2 of a length-N transform: the pair with the
 // smallest max(N1, N2) (threads per vector are max(N1, N2), so a lopsided
-// split idles most of them in one pass), N1 in {16, 12, 9, 8, 6, 4, 3, 2},
-// N2 <= 24 and 3-smooth; ties keep the larger N1.
+// split idles most of them in one pass), N1 in {16, 12, 9, 8, 6, 4, 3, 2, 18},
+// N2 <= 24 and 3-smooth; ties keep the first.
 constexpr bool smooth23(int n)
 {
     while (n % 2 == 0) n /= 2;
@@ -179,9 +179,9 @@ constexpr bool smooth23(int n)
 constexpr int plan2_n1(int N)
 {
     if (N == 24) return 8;  // 8 x 3: the z outputs kept are whole blocks of the second pass
-    const int cand[8] = {16, 12, 9, 8, 6, 4, 3, 2};
+    const int cand[9] = {16, 12, 9, 8, 6, 4, 3, 2, 18};
     int best = 1, score = N;
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < 9; k++) {
         const int c = cand[k];
         if (N % c != 0 || N / c > 24 || !smooth23(N / c)) continue;
         const int sc = c > N / c ? c : N / c;
@@ -209,6 +209,7 @@ struct FastDiv {
 };
 
 // Sizes with a compiled fast path (Ngal = 3N/2 of the usual channel grids).
-#define LH_FAST_SIZES(X) X(12) X(24) X(48) X(96) X(144) X(192) X(288) X(384)
+#define LH_FAST_SIZES(X) \
+    X(12) X(24) X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(162) X(192) X(216) X(288) X(324) X(384)
 
 }  // namespace lh

@@ -38,20 +38,16 @@
 #ifndef LH_ZFWD_B
 #define LH_ZFWD_B 3
 #endif
-// The block-synchronous kernels at the large lengths hold longer register
-// FFTs (18 and 24 threads per vector at Ngal 288 and 384): at three CTAs per
-// SM (80 registers) they spilled 0.1-0.8 KB per thread.  From LH_LARGE_N on,
-// the bound is LH_LARGE_B CTAs per SM (128 registers, no spills).  Measured
-// on B200 (ms per RK3 step): 256^2 x 257 12.32 -> 10.15; 192^2 x 257 5.04 ->
-// 4.88, x 153 3.11 -> 3.01, x 97 2.00 -> 1.93 (with one z row per x CTA; with
-// three it lost 1 %); at Ngal 192 two CTAs lost in the step graph.
-#ifndef LH_LARGE_N
-#define LH_LARGE_N 288
-#endif
+// The z kernels at the lengths of 18 and more threads per vector hold longer
+// register FFTs: at three CTAs per SM (80 registers) they spilled 0.1-0.8 KB per
+// thread.  There the bound is LH_LARGE_B CTAs per SM (128 registers, no spills).
+// Measured on B200 (ms per RK3 step): 256^2 x 257 12.32 -> 10.15; 192^2 x 257
+// 5.04 -> 4.88, x 153 3.11 -> 3.01, x 97 2.00 -> 1.93; at Ngal 192 two CTAs lost
+// in the step graph.
 #ifndef LH_LARGE_B
 #define LH_LARGE_B 2
 #endif
-#define LH_MINB(N, B) ((N) >= LH_LARGE_N ? LH_LARGE_B : (B))
+#define LH_MINB(N, B) (Plan2<N>::N1 >= 18 || Plan2<N>::N2 >= 18 ? LH_LARGE_B : (B))
 #include "lh_kernels.cuh"
 #include "lh_xprod.cuh"
 
@@ -200,7 +196,7 @@ __global__ void __launch_bounds__(LH_ZINV_T, LH_ZINV_B) k_zinv_w(const Inst *__r
 // Four CTAs an SM (128 registers) spill: 372 us at 128^2, 1764 at 192^2; three
 // instead of two at Mx = 384 3150.
 template <int NX>
-__global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 9 ? 4 : (XPlan<NX>::N2 <= 18 ? 3 : 2))
+__global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 6 ? 4 : (XPlan<NX>::N2 <= 18 ? 3 : 2))
     k_xprod_r(const Inst *__restrict__ insts, const Work *__restrict__ work, int rb, int want_max)
 {
     using XP = XPlan<NX>;
@@ -208,10 +204,12 @@ __global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 9 ? 4 : (XPlan
     extern __shared__ double2 sm[];
     const Work w = work[blockIdx.x];
     const Inst &I = insts[w.inst];
-    const int t = threadIdx.x, r = t % XP::N1, row = t / XP::N1;
+    const int lane = threadIdx.x & 31, r = lane % XP::N1;
+    const bool on = lane < XP::RW * XP::N1;
+    const int row = (threadIdx.x >> 5) * XP::RW + (on ? lane / XP::N1 : 0);
     const int Mz = I.Mz, j = w.j;
     const int q = w.blk * rb + row;  // this lane's z row
-    const bool rowok = row < rb && q < Mz;
+    const bool rowok = on && row < rb && q < Mz;
     // this row in the planes the y interpolations read
     const size_t fs = (size_t)Mz * nxh, orow = (size_t)min(q, Mz - 1) * nxh;
     const double2 *u1j = sin_field(I, w.aux + 1, 0) + orow, *u3j = u1j + fs, *vj = u3j + fs;
@@ -224,7 +222,7 @@ __global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 9 ? 4 : (XPlan
     const bool track = want_max && I.dt_mode == 0 && j <= I.nyu - 1;  // maxima over planes 1..nyu-1
     double m1 = 0.0, m3 = 0.0;
     xrow<NX>(
-        sm + (size_t)row * XP::N1 * XP::LD, I.twx, r, rowok, track, m1, m3,
+        sm + (size_t)row * XP::N1 * XP::LD, I.twx, r, on, rowok, track, m1, m3,
         [&](int pair, const int *k, double2 *A, double2 *B) {
             if (pair == 0) {  // (u1, u3) at the centre
 #pragma unroll

@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_plane_small(const Inst *__
             double2 *const row = P + (rowok ? z : 0) * LDX;
             double2 FA[XP::KQ], FB[XP::KQ];  // (u1, u3) at the face, interpolated before pair 0's products take its slots
             xrow<NX>(
-                T, I.twx, r, rowok, track, m1, m3,
+                T, I.twx, r, true, rowok, track, m1, m3,
                 [&](int pair, const int *k, double2 *A, double2 *B) {
                     if (pair == 0) {
 #pragma unroll

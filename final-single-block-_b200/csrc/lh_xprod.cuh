@@ -64,12 +64,18 @@ template <int NX>
 struct XPlan {
     // the substep at the other splits, us: 192 as 8 x 24 394 (16 x 12: 362), 144 as
     // 8 x 18 153 (148), 96 as 4 x 24 129 and 16 x 6 123 (114), 48 as 4 x 12 51 (44)
-    static constexpr int N1 = NX == 12 ? 4 : (NX <= 96 ? 8 : 16);
+    static constexpr int N1 = NX == 12                                         ? 4
+                              : (NX == 36 || NX == 54 || NX == 162)            ? 6
+                              : (NX == 24 || NX == 48 || NX == 72 || NX == 96) ? 8
+                              : (NX == 108 || NX == 216 || NX == 324)          ? 12
+                                                                               : 16;
     static constexpr int N2 = NX / N1;
     static constexpr int LD = N2 | 1;             // odd row stride: conflict-free rows and columns
     static constexpr int KQ = NX / 3 / N2 + 1;    // modes k <= Nx/2 of a task, at most
     static constexpr int ROUNDS = N2 <= N1 ? 1 : ((N2 + 1) / 2 + N1 / 2 - 1) / (N1 / 2);
-    static constexpr int RW = 32 / N1;            // rows per warp
+    static constexpr int RW = 32 / N1;            // rows per warp; N1 = 6 and 12 leave lanes over
+    static constexpr bool WHOLE = RW * N1 == 32;
+    static_assert(N1 * N2 == NX && N1 % 2 == 0 && 2 * KQ <= N1 + 1, "modes, mirror images, zeros between");
 };
 // Task of lane r in round g and the lane that holds task N2 - m; -1: idle.
 // Round 0: m = 0 .. N1/2 - 1, N2/2, and the mirror images N2 - m downwards from
@@ -94,9 +100,10 @@ __device__ __forceinline__ void xtask(int g, int r, int &m, int &partner)
 // The three pairs of a row: load(pair, k, A, B) fetches the modes k[] of the two
 // real rows, store(pair, k, A, B) takes the spectra of the two products at mode k.
 // T: the row's exchange matrix; r: this lane of the row's N1; m1, m3 gather max
-// |u1|, |u3| when track.  Every lane of the warp calls it (rowok = false: idle).
+// |u1|, |u3| when track.  Every lane of the warp calls it, with rowok = false
+// past the rows and on = false on the lanes left over.
 template <int NX, class Load, class Store>
-__device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int r, bool rowok, bool track, double &m1,
+__device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int r, bool on, bool rowok, bool track, double &m1,
                                      double &m3, Load &&load, Store &&store)
 {
     using XP = XPlan<NX>;
@@ -140,7 +147,7 @@ __device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int r, bool 
                 a[N1 - 1 - n1] = n2 == 0 ? own : z;
             }
             DFT<N1, +1, NX>::run(a, tw);
-            if (n2 >= 0) {
+            if (n2 >= 0 && (XP::WHOLE || on)) {
                 TwStep ts(__ldg(tw + n2));
 #pragma unroll
                 for (int k1 = 0; k1 < N1; k1++) T[k1 * LD + n2] = k1 > 0 ? twiddle<+1>(ts.next(), a[k1]) : a[k1];
@@ -178,7 +185,10 @@ __device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int r, bool 
             DFT<N2, -1, NX>::run(b, tw);
             TwStep ts(__ldg(tw + r));
 #pragma unroll
-            for (int m = 0; m < N2; m++) T[r * LD + m] = m > 0 ? twiddle<-1>(ts.next(), b[m]) : b[m];
+            for (int m = 0; m < N2; m++) {
+                const double2 z = m > 0 ? twiddle<-1>(ts.next(), b[m]) : b[m];
+                if (XP::WHOLE || on) T[r * LD + m] = z;
+            }
         }
         __syncwarp();
         // forward pass 2, split, scale 1/Mx

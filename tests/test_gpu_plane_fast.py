@@ -9,7 +9,8 @@ from helpers import rel_l2
 pytestmark = pytest.mark.gpu
 
 # Nx, Nz: transform lengths 3N/2 in x and z
-SIZES = [(8, 8), (16, 8), (8, 16), (32, 16), (64, 16), (96, 8), (128, 8), (192, 16), (256, 8), (16, 96), (8, 192), (16, 256)]
+SIZES = [(8, 8), (16, 8), (8, 16), (32, 16), (64, 16), (96, 8), (128, 8), (192, 16), (256, 8), (16, 96), (8, 192), (16, 256),
+         (24, 24), (36, 48), (48, 36), (72, 24), (108, 16), (144, 16), (216, 8), (8, 72), (16, 108), (8, 144), (24, 216)]
 
 
 @pytest.mark.parametrize("Nx,Nz", SIZES)
