@@ -718,6 +718,23 @@ __global__ void k_plane_to_col(const double2 *__restrict__ src, double2 *__restr
     }
 }
 
+// The same for a real matrix (spectra accumulators): plane-major rows to
+// out[column][row].
+__global__ void k_rows_to_cols(const double *__restrict__ src, double *__restrict__ dst, int len, int nc)
+{
+    __shared__ double tile[32][33];
+    const int c0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+        const int j = j0 + r, c = c0 + threadIdx.x;
+        if (c < nc && j < len) tile[r][threadIdx.x] = src[(size_t)j * nc + c];
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+        const int c = c0 + r, j = j0 + threadIdx.x;
+        if (c < nc && j < len) dst[(size_t)c * len + j] = tile[threadIdx.x][r];
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Stand-alone LUsolU on plane-major columns (unit entry): grid 2 = u/w
 // (rows 0..nyu+1), 1 = v (rows 0..nyv+1)

@@ -33,6 +33,7 @@ __global__ void k_column_bcd(const Inst *__restrict__ insts, const Work *__restr
 __global__ void k_dt(const Inst *__restrict__ insts, int ninst);
 __global__ void k_col_to_plane(const double2 *__restrict__ src, double2 *__restrict__ dst, int len, int nc);
 __global__ void k_plane_to_col(const double2 *__restrict__ src, double2 *__restrict__ dst, int len, int nc);
+__global__ void k_rows_to_cols(const double *__restrict__ src, double *__restrict__ dst, int len, int nc);
 __global__ void k_lusolu(const Inst *__restrict__ insts, int grid, int kRK, double dt, const double2 *rhs,
                          double2 *u, double *fac);
 __global__ void k_lusolp(const Inst *__restrict__ insts, double2 *x);
