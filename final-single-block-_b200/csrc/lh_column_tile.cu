@@ -619,6 +619,112 @@ __global__ void __launch_bounds__(kTileBlocks *C, 8 / C) k_column_tile(const Ins
     }
 }
 
+// ---------------------------------------------------------------------------
+// LUsolU (tridLU_3D.f90:38-94, with LU_build + LU_dec) on plane-major columns,
+// 32 lanes to a column, K rows a lane in registers, so the right-hand side is
+// read once and the solution written once (in place too: a CTA has read its
+// columns before it writes them).  Pivots and substitutions as in the tiles:
+// composed maps, entries, then the reference's rows.  One lane a column
+// (k_lusolu) waits on its loads row by row in two sweeps and keeps the factors
+// in global memory in between.  Bound by HBM and, at the 8 columns of a CTA, by
+// the latency of the scans: 41 MB at 128x128x153, 57 -> 21 us a call on B200.
+template <int K>
+__global__ void __launch_bounds__(kTileBlocks * 8) k_lusolu_tile(const Inst *__restrict__ insts, int grid, int kRK,
+                                                                 double dt, const double2 *rhs, double2 *u)
+{
+    constexpr int C = 8, T = kTileBlocks * C;
+    extern __shared__ double sd[];  // the grid's d2/dy2 coefficients
+    __shared__ Mob maps[T];
+    __shared__ Aff<1> part[2][kTileBlocks / 4 * C];
+    const Inst &I = insts[0];
+    const int t = threadIdx.x, c = t % C, b = t / C, nc = I.nc, nxh = I.nxh;
+    const int n = grid == 2 ? I.nyu : I.nyv;  // rows 0..n+1
+    const int col = blockIdx.x * C + c, cc = min(col, nc - 1), r0 = b * K;
+    double2 r[K];
+#pragma unroll
+    for (int q = 0; q < K; q++) r[q] = rhs[(size_t)min(r0 + q, n + 1) * nc + cc];
+    const double *d = grid == 2 ? I.dyu2i : I.dyv2i;
+    for (int e = t; e < 3 * (n + 1); e += T) sd[e] = d[e];
+    const double k2x = I.k2x[cc % nxh], k2z = I.k2z[cc / nxh];
+    const double beta = rk_coeffs(kRK).b * dt / I.Re;
+    const double w0 = grid == 2 ? I.gw1 : 0.0, wt = grid == 2 ? I.gw2 : 0.0;
+    __syncthreads();
+    // pivots
+    Mob m{1.0, 0.0, 0.0, 1.0};
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        if (r0 + q > n + 1) continue;
+        const HRow h = helm_row(r0 + q, n, sd, beta, k2x, k2z, w0, wt);
+        m = Mob{h.a3 * m.c, h.a3 * m.d, fma(h.a2, m.c, -h.a1 * m.a), fma(h.a2, m.d, -h.a1 * m.b)};
+    }
+    mob_rescale(m);
+    maps[t] = m;
+    __syncthreads();
+    double p = 0.0, s = 1.0;  // the entering scaled diagonal as p / s (row 0 ignores it)
+#pragma unroll 4
+    for (int k = c; k < t; k += C) {
+        const Mob f = maps[k];
+        const double x = fma(f.a, p, f.b * s);
+        s = fma(f.c, p, f.d * s);
+        p = x;
+    }
+    double x = p / s, iv[K];
+    Aff<1> a;
+    a.reset();
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        if (r0 + q > n + 1) continue;
+        const HRow h = helm_row(r0 + q, n, sd, beta, k2x, k2z, w0, wt);
+        iv[q] = 1.0 / (h.a2 - h.a1 * x);
+        x = h.a3 * iv[q];
+        a.A[0] = make_double2((r[q].x - h.a1 * a.A[0].x) * iv[q], (r[q].y - h.a1 * a.A[0].y) * iv[q]);
+        a.B[0] = -(h.a1 * iv[q]) * a.B[0];
+    }
+    double2 y = scan_entry<C, 1>(a, part[0], true).A[0];
+    a.reset();
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        if (r0 + q > n + 1) continue;
+        const HRow h = helm_row(r0 + q, n, sd, beta, k2x, k2z, w0, wt);
+        y = make_double2((r[q].x - h.a1 * y.x) * iv[q], (r[q].y - h.a1 * y.y) * iv[q]);
+        r[q] = y;
+        iv[q] = h.a3 * iv[q];  // the scaled upper diagonal
+        a.A[0] = a.at(0, y);
+        a.B[0] = -iv[q] * a.B[0];
+    }
+    double2 v = scan_entry<C, 1>(a, part[1], false).A[0];
+#pragma unroll
+    for (int q = K - 1; q >= 0; q--) {
+        if (r0 + q > n + 1) continue;
+        v = make_double2(r[q].x - iv[q] * v.x, r[q].y - iv[q] * v.y);
+        if (col < nc) u[(size_t)(r0 + q) * nc + col] = v;
+    }
+}
+
+// Loads every kernel lusolu_launch may pick on the current device, so that none
+// is loaded for the first time inside a stream capture.
+cudaError_t lusolu_load()
+{
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, (const void *)k_lusolu_tile<5>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void *)k_lusolu_tile<9>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void *)k_lusolu);
+    return e;
+}
+
+// LUsolU of every column; fac: scratch of rows x columns for columns too tall
+// for the lanes' registers.
+void lusolu_launch(const Inst *insts, int grid, int kRK, double dt, int rows, int nc, const double2 *rhs, double2 *u,
+                   double *fac, cudaStream_t st)
+{
+    const unsigned blocks = (unsigned)((nc + 7) / 8);
+    const size_t smem = 3 * (size_t)rows * sizeof(double);
+    if (rows <= 5 * kTileBlocks) k_lusolu_tile<5><<<blocks, kTileBlocks * 8, smem, st>>>(insts, grid, kRK, dt, rhs, u);
+    else if (rows <= 9 * kTileBlocks)
+        k_lusolu_tile<9><<<blocks, kTileBlocks * 8, smem, st>>>(insts, grid, kRK, dt, rhs, u);
+    else k_lusolu<<<(nc + 127) / 128, 128, 0, st>>>(insts, grid, kRK, dt, rhs, u, fac);
+}
+
 cudaError_t column_tile_attributes(int C, size_t smem)
 {
     return raise_smem_limit(C == 8 ? (const void *)k_column_tile<8>

@@ -36,6 +36,10 @@ __global__ void k_plane_to_col(const double2 *__restrict__ src, double2 *__restr
 __global__ void k_rows_to_cols(const double *__restrict__ src, double *__restrict__ dst, int len, int nc);
 __global__ void k_lusolu(const Inst *__restrict__ insts, int grid, int kRK, double dt, const double2 *rhs,
                          double2 *u, double *fac);
+// the same without global scratch where the rows fit the lanes (lh_column_tile.cu)
+void lusolu_launch(const Inst *insts, int grid, int kRK, double dt, int rows, int nc, const double2 *rhs, double2 *u,
+                   double *fac, cudaStream_t st);
+cudaError_t lusolu_load();
 __global__ void k_lusolp(const Inst *__restrict__ insts, double2 *x);
 __global__ void k_divmax(const Inst *__restrict__ insts, double *out);
 

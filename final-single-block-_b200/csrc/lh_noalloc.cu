@@ -7,7 +7,8 @@
 // whose device memory is owned by another allocator.  lh_lusolu_noalloc()
 // takes the right-hand side and the solution as device arrays the caller
 // already owns and keeps its only scratch -- one scaled upper diagonal per
-// row and column -- in the file-scope array below.
+// row and column, where the columns are too tall to be solved in registers --
+// in the file-scope array below.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -42,6 +43,7 @@ cudaError_t scratch_on_current_device(double **out)
     if (!g_scratch_addr[dev]) {
         double *p = nullptr;
         e = cudaGetSymbolAddress((void **)&p, g_lusolu_scratch);
+        if (e == cudaSuccess) e = lh::lusolu_load();
         if (e != cudaSuccess) return e;
         g_scratch_addr[dev] = p;
     }
@@ -87,9 +89,8 @@ extern "C" int lh_lusolu_noalloc(lh_ctx *c, int grid, int kRK, double dt, const 
         c->err = std::string("lh_lusolu_noalloc: earlier error on this thread: ") + cudaGetErrorString(e);
         return LH_ECUDA;
     }
-    lh::k_lusolu<<<(s.nc + 127) / 128, 128, 0, c->st>>>(c->d_inst, grid, kRK, dt,
-                                                       reinterpret_cast<const double2 *>(rhs_dev),
-                                                       reinterpret_cast<double2 *>(u_dev), scratch);
+    lh::lusolu_launch(c->d_inst, grid, kRK, dt, (int)len, s.nc, reinterpret_cast<const double2 *>(rhs_dev),
+                      reinterpret_cast<double2 *>(u_dev), scratch, c->st);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         c->err = std::string("lh_lusolu_noalloc: launch: ") + cudaGetErrorString(e);

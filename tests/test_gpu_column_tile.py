@@ -45,3 +45,24 @@ def test_tiles_match_the_sequential_pass(Nx, Nz, ny, ctpress, cfl, monkeypatch):
         # mpgx: a flow-rate difference over dt; its terms agree to the last bit
         assert abs(out[1][1][k] - out[0][1][k]) <= 1e-10 * abs(out[0][1][k]), k
     assert out[1][2] < 1e-11
+
+
+@pytest.mark.parametrize("Nx,Nz,ny,grid", [(16, 4, 5, 2), (8, 18, 32, 1), (32, 18, 159, 2), (32, 18, 160, 2), (32, 18, 161, 1),
+                                           (32, 18, 287, 2), (16, 4, 288, 2)])
+def test_noalloc_solve_at_the_row_limits(Nx, Nz, ny, grid):
+    """lh_lusolu_noalloc solves in registers up to 160 and 288 rows and through
+    its scratch above; columns that are no multiple of 8, fewer rows than lanes."""
+    import numpy as np
+    import torch
+    from lh_b200 import Desc, Engine
+    d = Desc(Nx=Nx, Nz=Nz, ny=ny, dt_mode=1, dt=5e-3)
+    e = Engine(d)
+    n = d.nyu + 2 if grid == 2 else d.nyv + 2
+    rng = np.random.default_rng(ny)
+    rhs = rng.standard_normal((d.ncols, n)) + 1j * rng.standard_normal((d.ncols, n))
+    want = e.lusolu(grid, 2, d.dt, rhs)
+    x = torch.from_numpy(np.ascontiguousarray(rhs.T)).to("cuda")
+    torch.cuda.synchronize()
+    assert e.L.lh_lusolu_noalloc(e.h, grid, 2, d.dt, x.data_ptr(), x.data_ptr()) == 0
+    e.synchronize()
+    assert rel_l2(x.cpu().numpy().T, want) <= 1e-13
