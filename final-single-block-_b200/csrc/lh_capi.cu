@@ -54,7 +54,9 @@ extern "C" int lh_ctx_create(const lh_grid_desc *desc, lh_ctx **out)
     }
     cudaError_t e = cudaGetDevice(&c->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMallocHost(&c->h_err, sizeof(int));
     if (e != cudaSuccess) {
+        if (c->st) cudaStreamDestroy(c->st);
         delete c;
         return LH_ECUDA;
     }
@@ -88,6 +90,7 @@ extern "C" int lh_ctx_destroy(lh_ctx *c)
     stats_release(c->stats_scr);
     instance_free(c->dev);
     if (c->st) cudaStreamDestroy(c->st);
+    if (c->h_err) cudaFreeHost(c->h_err);
     delete c;
     return LH_OK;
 }
@@ -161,12 +164,13 @@ extern "C" int lh_download_nu(lh_ctx *c, double *nu1, double *nu2, double *nu3)
     return LH_OK;
 }
 
+// Waits for the stream and looks at the error word, which lands in page-locked
+// memory (a copy to pageable memory waits by itself).
 static int check_err_word(lh_ctx *c)
 {
-    int h = 0;
-    CK(cudaMemcpyAsync(&h, c->dev.inst.err, sizeof(int), cudaMemcpyDeviceToHost, c->st), "error word");
+    CK(cudaMemcpyAsync(c->h_err, c->dev.inst.err, sizeof(int), cudaMemcpyDeviceToHost, c->st), "error word");
     CK(cudaStreamSynchronize(c->st), "synchronize");
-    if (h & ERR_NONFINITE) return fail(c, LH_EDEVICE, "non-finite values in the state (time step unstable?)");
+    if (*c->h_err & ERR_NONFINITE) return fail(c, LH_EDEVICE, "non-finite values in the state (time step unstable?)");
     return LH_OK;
 }
 
@@ -258,7 +262,6 @@ extern "C" int lh_step_host(lh_ctx *c, double *u1, double *u2, double *u3, doubl
 extern "C" int lh_synchronize(lh_ctx *c)
 {
     if (!c) return LH_EINVAL;
-    CK(cudaStreamSynchronize(c->st), "synchronize");
     return check_err_word(c);
 }
 
@@ -488,8 +491,14 @@ extern "C" int lh_lusolu(lh_ctx *c, int grid, int kRK, double dt, const double *
     if (e == cudaSuccess) e = cudaMalloc(&d_f, n * sizeof(double));
     if (e == cudaSuccess) e = cudaMemcpyAsync(c->dev.stage, rhs, n * sizeof(double2), cudaMemcpyHostToDevice, c->st);
     if (e == cudaSuccess) {
-        dim3 g((s.nc + 31) / 32, (len + 31) / 32), b(32, 8);
-        k_col_to_plane<<<g, b, 0, c->st>>>(c->dev.stage, d_r, len, s.nc);
+        FieldSet f;
+        f.src[0] = c->dev.stage;
+        f.dst[0] = d_r;
+        f.len[0] = len;
+        f.nc = s.nc;
+        e = cols_to_planes(f, 1, c->st);
+    }
+    if (e == cudaSuccess) {
         k_lusolu<<<(s.nc + 127) / 128, 128, 0, c->st>>>(c->d_inst, grid, kRK, dt, d_r, d_u, d_f);
         e = cudaGetLastError();
     }
@@ -512,8 +521,14 @@ extern "C" int lh_lusolp(lh_ctx *c, double *x)
     CK(cudaMalloc(&d_x, n * sizeof(double2)), "alloc");
     cudaError_t e = cudaMemcpyAsync(c->dev.stage, x, n * sizeof(double2), cudaMemcpyHostToDevice, c->st);
     if (e == cudaSuccess) {
-        dim3 g((s.nc + 31) / 32, (len + 31) / 32), b(32, 8);
-        k_col_to_plane<<<g, b, 0, c->st>>>(c->dev.stage, d_x, len, s.nc);
+        FieldSet f;
+        f.src[0] = c->dev.stage;
+        f.dst[0] = d_x;
+        f.len[0] = len;
+        f.nc = s.nc;
+        e = cols_to_planes(f, 1, c->st);
+    }
+    if (e == cudaSuccess) {
         k_lusolp<<<(s.nc + 127) / 128, 128, 0, c->st>>>(c->d_inst, d_x);
         e = cudaGetLastError();
     }

@@ -688,34 +688,93 @@ __global__ void k_dt(const Inst *__restrict__ insts, int ninst)
 // Layout transforms between the reference column layout x(j, column) (j
 // fastest) and the plane-major device layout [j][column]: a 32x32 tiled
 // transpose of a len x nc complex matrix.
-__global__ void k_col_to_plane(const double2 *__restrict__ src, double2 *__restrict__ dst, int len, int nc)
+// One launch moves up to four fields (blockIdx.z).  The column side may be page-locked
+// host memory: every access to it is 16 bytes a lane, 512 contiguous a warp, and a
+// thread has its four loads in flight at once.  A null source gives zeros.
+__global__ void k_cols_to_planes(const FieldSet f)
 {
     __shared__ double2 tile[32][33];
+    const double2 *__restrict__ src = f.src[blockIdx.z];
+    double2 *__restrict__ dst = f.dst[blockIdx.z];
+    const int len = f.len[blockIdx.z], nc = f.nc;
     const int c0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int c = c0 + r, j = j0 + threadIdx.x;
-        if (c < nc && j < len) tile[r][threadIdx.x] = src[(size_t)c * len + j];
+    double2 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int c = c0 + threadIdx.y + 8 * q, j = j0 + threadIdx.x;
+        v[q] = make_double2(0.0, 0.0);
+        if (src && c < nc && j < len) v[q] = src[(size_t)c * len + j];
     }
+#pragma unroll
+    for (int q = 0; q < 4; q++) tile[threadIdx.y + 8 * q][threadIdx.x] = v[q];
     __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int j = j0 + r, c = c0 + threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int r = threadIdx.y + 8 * q, j = j0 + r, c = c0 + threadIdx.x;
         if (c < nc && j < len) dst[(size_t)j * nc + c] = tile[threadIdx.x][r];
     }
 }
 
-__global__ void k_plane_to_col(const double2 *__restrict__ src, double2 *__restrict__ dst, int len, int nc)
+__global__ void k_planes_to_cols(const FieldSet f)
 {
     __shared__ double2 tile[32][33];
+    const double2 *__restrict__ src = f.src[blockIdx.z];
+    double2 *__restrict__ dst = f.dst[blockIdx.z];
+    const int len = f.len[blockIdx.z], nc = f.nc;
     const int c0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int j = j0 + r, c = c0 + threadIdx.x;
-        if (c < nc && j < len) tile[r][threadIdx.x] = src[(size_t)j * nc + c];
+    double2 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int j = j0 + threadIdx.y + 8 * q, c = c0 + threadIdx.x;
+        v[q] = make_double2(0.0, 0.0);
+        if (c < nc && j < len) v[q] = src[(size_t)j * nc + c];
     }
+#pragma unroll
+    for (int q = 0; q < 4; q++) tile[threadIdx.y + 8 * q][threadIdx.x] = v[q];
     __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int c = c0 + r, j = j0 + threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int r = threadIdx.y + 8 * q, c = c0 + r, j = j0 + threadIdx.x;
         if (c < nc && j < len) dst[(size_t)c * len + j] = tile[threadIdx.x][r];
     }
+}
+
+static dim3 field_grid(const FieldSet &f, int n)
+{
+    int len = 1;
+    for (int k = 0; k < n; k++) len = f.len[k] > len ? f.len[k] : len;
+    return dim3((f.nc + 31) / 32, (len + 31) / 32, n);
+}
+
+cudaError_t cols_to_planes(const FieldSet &f, int n, cudaStream_t st)
+{
+    k_cols_to_planes<<<field_grid(f, n), dim3(32, 8), 0, st>>>(f);
+    return cudaGetLastError();
+}
+
+cudaError_t planes_to_cols(const FieldSet &f, int n, cudaStream_t st)
+{
+    k_planes_to_cols<<<field_grid(f, n), dim3(32, 8), 0, st>>>(f);
+    return cudaGetLastError();
+}
+
+// What an upload sets beside the fields (getini): Nu = 0 before the first step
+// (littleharsh.f90:127-129), the scalars and the error word.
+__global__ void k_reset_state(const StateReset r)
+{
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    for (size_t q = t; q < r.n; q += step) r.nu1[q] = r.nu2[q] = r.nu3[q] = make_double2(0.0, 0.0);
+    if (t == 0) {
+#pragma unroll
+        for (int k = 0; k < SC_COUNT; k++) r.sc[k] = r.value[k];
+        *r.err = 0;
+    }
+}
+
+cudaError_t reset_state(const StateReset &r, cudaStream_t st)
+{
+    k_reset_state<<<(unsigned)(r.n / 1024 < 296 ? r.n / 1024 + 1 : 296), 256, 0, st>>>(r);
+    return cudaGetLastError();
 }
 
 // The same for a real matrix (spectra accumulators): plane-major rows to

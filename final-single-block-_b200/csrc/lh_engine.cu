@@ -2,7 +2,10 @@
 // the host boundary, work tables and the launch sequence of a substep.
 #include "lh_engine.h"
 
+#include <cuda.h>
+
 #include <algorithm>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -213,58 +216,134 @@ void instance_free(DevInstance &d)
     d.block = nullptr;
 }
 
-static cudaError_t upload_field(DevInstance &d, const double *src, double2 *dst, int len, cudaStream_t st)
+// Transfers of at most this many bytes between page-locked host buffers and the
+// device are one kernel that reads or writes the host buffers itself instead of a
+// copy and a transform per field through the staging field.  Two transfers of four
+// fields on B200, copies / kernel, us: 136 columns x 98 rows (0.9 MB) up 56 / 26,
+// down 54 / 25; 528 x 154 (5 MB) 134 / 116, 146 / 111; 2080 x 154 (20 MB) 428 / 431,
+// 415 / 410; 8256 x 154 (81 MB) 1542 / 1684, 1486 / 1660, where the copy engine's
+// larger packets win.
+constexpr size_t kDirectBytes = (size_t)16 << 20;
+
+// Whether the device may access [p, p + bytes) of host memory in place: one
+// page-locked allocation or registration that holds all of it, visible under the
+// same address, aligned for double2 accesses and not read-only or device I/O.
+static bool direct_host(const void *p, size_t bytes)
+{
+    using GetAttribute = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    static const GetAttribute get = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return (GetAttribute)f;
+    }();
+    cudaPointerAttributes a;
+    unsigned flags = 0;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    if (!get || ((uintptr_t)p & 15) != 0) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (a.type != cudaMemoryTypeHost || a.devicePointer != p) return false;
+    if (cudaHostGetFlags(&flags, const_cast<void *>(p)) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (flags & (cudaHostRegisterIoMemory | cudaHostRegisterReadOnly)) return false;
+    if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)p) != CUDA_SUCCESS ||
+        get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)p) != CUDA_SUCCESS)
+        return false;
+    return (CUdeviceptr)p >= start && (CUdeviceptr)p + bytes <= start + size;
+}
+
+// The host side of n fields (null entries move nothing); fields that share memory
+// are left to the copies, which keep their order.
+static bool direct_transfer(const void *const *host, const int *len, int n, int nc)
+{
+    size_t total = 0;
+    for (int k = 0; k < n; k++) total += host[k] ? (size_t)len[k] * nc * sizeof(double2) : 0;
+    if (total > kDirectBytes) return false;
+    for (int k = 0; k < n; k++) {
+        const size_t bk = (size_t)len[k] * nc * sizeof(double2);
+        if (!host[k]) continue;
+        for (int q = 0; q < k; q++) {
+            const size_t bq = (size_t)len[q] * nc * sizeof(double2);
+            if (host[q] && (uintptr_t)host[k] < (uintptr_t)host[q] + bq && (uintptr_t)host[q] < (uintptr_t)host[k] + bk)
+                return false;
+        }
+        if (!direct_host(host[k], bk)) return false;
+    }
+    return true;
+}
+
+static cudaError_t upload_fields(DevInstance &d, const double *const *src, double2 *const *dst, const int *len, int n,
+                                 cudaStream_t st)
 {
     const int nc = d.hs.nc;
-    if (!src) return cudaMemsetAsync(dst, 0, (size_t)len * nc * sizeof(double2), st);
-    cudaError_t e = cudaMemcpyAsync(d.stage, src, (size_t)len * nc * sizeof(double2), cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return e;
-    dim3 grid((nc + 31) / 32, (len + 31) / 32), block(32, 8);
-    k_col_to_plane<<<grid, block, 0, st>>>(d.stage, dst, len, nc);
-    return cudaGetLastError();
+    const bool direct = direct_transfer((const void *const *)src, len, n, nc);
+    FieldSet f;
+    f.nc = nc;
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < n && e == cudaSuccess; k++) {
+        const int q = direct ? k : 0;
+        f.src[q] = direct ? (const double2 *)src[k] : d.stage;
+        f.dst[q] = dst[k];
+        f.len[q] = len[k];
+        if (direct) continue;
+        const size_t bytes = (size_t)len[k] * nc * sizeof(double2);
+        if (!src[k]) {
+            e = cudaMemsetAsync(dst[k], 0, bytes, st);
+        } else {
+            e = cudaMemcpyAsync(d.stage, src[k], bytes, cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess) e = cols_to_planes(f, 1, st);
+        }
+    }
+    if (direct) e = cols_to_planes(f, n, st);
+    return e;
 }
 
 cudaError_t download_field(const DevInstance &d, const double2 *src, int len, double *dst, cudaStream_t st)
 {
-    const int nc = d.hs.nc;
-    dim3 grid((nc + 31) / 32, (len + 31) / 32), block(32, 8);
-    k_plane_to_col<<<grid, block, 0, st>>>(src, d.stage, len, nc);
-    cudaError_t e = cudaGetLastError();
+    FieldSet f;
+    f.nc = d.hs.nc;
+    f.src[0] = src;
+    f.dst[0] = d.stage;
+    f.len[0] = len;
+    cudaError_t e = planes_to_cols(f, 1, st);
     if (e != cudaSuccess) return e;
-    return cudaMemcpyAsync(dst, d.stage, (size_t)len * nc * sizeof(double2), cudaMemcpyDeviceToHost, st);
+    return cudaMemcpyAsync(dst, d.stage, (size_t)len * f.nc * sizeof(double2), cudaMemcpyDeviceToHost, st);
 }
 
-// The fields but p, the Nu reset and the scalars of an upload (getini).
-static cudaError_t upload_without_p(DevInstance &d, const double *u1, const double *u2, const double *u3,
-                                    cudaStream_t st)
+// The Nu reset and the scalars of an upload (getini).
+static cudaError_t upload_scalars(DevInstance &d, const double *u1, cudaStream_t st)
 {
     const HostSetup &s = d.hs;
     Inst &I = d.inst;
-    cudaError_t e;
-    if ((e = upload_field(d, u1, I.U1, s.nyu + 2, st)) != cudaSuccess) return e;
-    if ((e = upload_field(d, u2, I.U2, s.nyv + 2, st)) != cudaSuccess) return e;
-    if ((e = upload_field(d, u3, I.U3, s.nyu + 2, st)) != cudaSuccess) return e;
-    const size_t npc = (size_t)s.nyu * s.nc * sizeof(double2);
-    // Nu = 0 before the first step (littleharsh.f90:127-129)
-    if ((e = cudaMemsetAsync(I.NU1, 0, npc, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(I.NU2, 0, npc, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(I.NU3, 0, npc, st)) != cudaSuccess) return e;
-    double sc[SC_COUNT] = {0};
-    sc[SC_T] = 0.0;
-    sc[SC_DT] = d.desc.dt_mode == LH_DT_FIXED ? d.desc.dt : 0.0;
-    sc[SC_MPGX] = d.desc.mpgx;
+    StateReset r{I.NU1, I.NU2, I.NU3, (size_t)s.nyu * s.nc, I.sc, I.err, {0}};
+    r.value[SC_T] = 0.0;
+    r.value[SC_DT] = d.desc.dt_mode == LH_DT_FIXED ? d.desc.dt : 0.0;
+    r.value[SC_MPGX] = d.desc.mpgx;
     const double q = u1 ? flowrate_host(s, u1) : 0.0;
-    sc[SC_QX] = q;
-    sc[SC_QXT] = q;  // getini: QxT = Qx for the constant flow-rate mode
-    if ((e = cudaMemcpyAsync(I.sc, sc, sizeof(sc), cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
-    return cudaMemsetAsync(I.err, 0, sizeof(int), st);
+    r.value[SC_QX] = q;
+    r.value[SC_QXT] = q;  // getini: QxT = Qx for the constant flow-rate mode
+    return reset_state(r, st);
 }
 
 cudaError_t instance_upload(DevInstance &d, const double *u1, const double *u2, const double *u3, const double *p,
                             cudaStream_t st)
 {
-    cudaError_t e = upload_without_p(d, u1, u2, u3, st);
-    if (e == cudaSuccess) e = upload_field(d, p, d.inst.P, d.hs.nyu, st);
+    const HostSetup &s = d.hs;
+    const double *src[4] = {u1, u2, u3, p};
+    double2 *dst[4] = {d.inst.U1, d.inst.U2, d.inst.U3, d.inst.P};
+    const int len[4] = {s.nyu + 2, s.nyv + 2, s.nyu + 2, s.nyu};
+    cudaError_t e = upload_scalars(d, u1, st);
+    if (e == cudaSuccess) e = upload_fields(d, src, dst, len, 4, st);
     if (e != cudaSuccess) return e;
     return cudaStreamSynchronize(st);
 }
@@ -272,9 +351,14 @@ cudaError_t instance_upload(DevInstance &d, const double *u1, const double *u2, 
 cudaError_t instance_upload_p_last(DevInstance &d, const double *u1, const double *u2, const double *u3,
                                    const double *p, cudaStream_t st, cudaEvent_t ev_u)
 {
-    cudaError_t e = upload_without_p(d, u1, u2, u3, st);
+    const HostSetup &s = d.hs;
+    const double *src[4] = {u1, u2, u3, p};
+    double2 *dst[4] = {d.inst.U1, d.inst.U2, d.inst.U3, d.inst.P};
+    const int len[4] = {s.nyu + 2, s.nyv + 2, s.nyu + 2, s.nyu};
+    cudaError_t e = upload_scalars(d, u1, st);
+    if (e == cudaSuccess) e = upload_fields(d, src, dst, len, 3, st);
     if (e == cudaSuccess) e = cudaEventRecord(ev_u, st);
-    if (e == cudaSuccess) e = upload_field(d, p, d.inst.P, d.hs.nyu, st);
+    if (e == cudaSuccess) e = upload_fields(d, src + 3, dst + 3, len + 3, 1, st);
     return e;
 }
 
@@ -282,11 +366,26 @@ cudaError_t instance_download(DevInstance &d, double *u1, double *u2, double *u3
 {
     const HostSetup &s = d.hs;
     const Inst &I = d.inst;
+    const double2 *src[4] = {I.U1, I.U2, I.U3, I.P};
+    double *dst[4] = {u1, u2, u3, p};
+    const int len[4] = {s.nyu + 2, s.nyv + 2, s.nyu + 2, s.nyu};
     cudaError_t e = cudaSuccess;
-    if (u1 && (e = download_field(d, I.U1, s.nyu + 2, u1, st)) != cudaSuccess) return e;
-    if (u2 && (e = download_field(d, I.U2, s.nyv + 2, u2, st)) != cudaSuccess) return e;
-    if (u3 && (e = download_field(d, I.U3, s.nyu + 2, u3, st)) != cudaSuccess) return e;
-    if (p && (e = download_field(d, I.P, s.nyu, p, st)) != cudaSuccess) return e;
+    if (direct_transfer((const void *const *)dst, len, 4, s.nc)) {
+        FieldSet f;
+        f.nc = s.nc;
+        int n = 0;
+        for (int k = 0; k < 4; k++) {
+            if (!dst[k]) continue;
+            f.src[n] = src[k];
+            f.dst[n] = (double2 *)dst[k];
+            f.len[n++] = len[k];
+        }
+        if (n) e = planes_to_cols(f, n, st);
+    } else {
+        for (int k = 0; k < 4 && e == cudaSuccess; k++)
+            if (dst[k]) e = download_field(d, src[k], len[k], dst[k], st);
+    }
+    if (e != cudaSuccess) return e;
     return cudaStreamSynchronize(st);
 }
 

@@ -31,8 +31,23 @@ __global__ void k_column(const Inst *__restrict__ insts, const Work *__restrict_
 __global__ void k_column_a(const Inst *__restrict__ insts, const Work *__restrict__ work, int kRK);
 __global__ void k_column_bcd(const Inst *__restrict__ insts, const Work *__restrict__ work, int kRK);
 __global__ void k_dt(const Inst *__restrict__ insts, int ninst);
-__global__ void k_col_to_plane(const double2 *__restrict__ src, double2 *__restrict__ dst, int len, int nc);
-__global__ void k_plane_to_col(const double2 *__restrict__ src, double2 *__restrict__ dst, int len, int nc);
+// layout transforms at the host boundary: n fields of len[k] x nc
+struct FieldSet {
+    const double2 *src[4] = {nullptr, nullptr, nullptr, nullptr};
+    double2 *dst[4] = {nullptr, nullptr, nullptr, nullptr};
+    int len[4] = {0, 0, 0, 0};
+    int nc = 0;
+};
+cudaError_t cols_to_planes(const FieldSet &f, int n, cudaStream_t st);
+cudaError_t planes_to_cols(const FieldSet &f, int n, cudaStream_t st);
+struct StateReset {
+    double2 *nu1, *nu2, *nu3;
+    size_t n;
+    double *sc;
+    int *err;
+    double value[SC_COUNT];
+};
+cudaError_t reset_state(const StateReset &r, cudaStream_t st);
 __global__ void k_rows_to_cols(const double *__restrict__ src, double *__restrict__ dst, int len, int nc);
 __global__ void k_lusolu(const Inst *__restrict__ insts, int grid, int kRK, double dt, const double2 *rhs,
                          double2 *u, double *fac);

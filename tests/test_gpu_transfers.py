@@ -1,0 +1,80 @@
+"""Host transfers: page-locked buffers the device reads and writes itself, buffers that
+go through the copies (pageable, off 16-byte alignment, shared by two fields, too
+large), and an upload's reset of Nu, scalars and the error word."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def buffers(shapes, kind):
+    import torch
+
+    keep, out = [], []
+    if kind == "shared":  # u3 and u1 in one buffer, u1 first: what a later field leaves stands
+        n = sum(2 * s[0] * s[1] for s in shapes)
+        big = torch.zeros(n, dtype=torch.float64).pin_memory().numpy()
+        o = 0
+        for s in shapes[:2] + [shapes[0]] + shapes[3:]:
+            out.append(big[o:o + 2 * s[0] * s[1]])
+            o += 2 * s[0] * s[1]
+        out[2] = out[0]
+        return out
+    for s in shapes:
+        n = 2 * s[0] * s[1]
+        if kind == "pageable":
+            out.append(np.zeros(n))
+        else:
+            t = torch.zeros(n + 1, dtype=torch.float64).pin_memory()
+            out.append(t.numpy()[1:] if kind == "odd" else t.numpy()[:n])
+    return out
+
+
+@pytest.mark.parametrize("N", [(12, 12, 33), (24, 16, 42), (32, 64, 65), (128, 128, 72)])
+@pytest.mark.parametrize("kind", ["pinned", "odd", "shared", "pageable"])
+def test_transfers(N, kind):
+    Nx, Nz, ny = N
+    from lh_b200 import Desc, Engine
+    from lh_b200.capi import _dp
+    c = Engine(Desc(Nx=Nx, Nz=Nz, ny=ny, dt_mode=1, dt=1e-4))
+    s = c.sizes
+    shapes = [(s.ncols, s.nyu + 2), (s.ncols, s.nyv + 2), (s.ncols, s.nyu + 2), (s.ncols, s.nyu)]
+    rng = np.random.default_rng(3)
+    want = [1e-3 * rng.standard_normal(2 * a * b) for a, b in shapes]
+    ref = [x.copy() for x in want]
+    bufs = buffers(shapes, kind)
+    def ck(rc):
+        c._ck(rc, "transfer")
+
+    for b, w in zip(bufs, want):
+        b[:] = w
+    if kind == "shared":  # one buffer takes u1 and then u3
+        ck(c.L.lh_upload_state(c.h, *[_dp(b) for b in want]))
+        want[0] = want[2]
+    else:
+        ck(c.L.lh_upload_state(c.h, *[_dp(b) for b in bufs]))
+    for b in bufs:
+        b[:] = -1.0
+    ck(c.L.lh_download_state(c.h, *[_dp(b) for b in bufs]))
+    for k, (b, w) in enumerate(zip(bufs, want)):
+        assert np.array_equal(b, w), k
+    # p left out: zeros; fields left out of a download stay as they are
+    ck(c.L.lh_upload_state(c.h, *[_dp(b) for b in bufs[:3]], None))
+    bufs[3][:] = 7.0
+    ck(c.L.lh_download_state(c.h, None, None, None, _dp(bufs[3])))
+    assert not bufs[3].any()
+    # the whole of a host step equals upload, step, download through pageable memory
+    if kind != "shared":
+        for b, w in zip(bufs, ref):
+            b[:] = w
+        ck(c.L.lh_step_host(c.h, *[_dp(b) for b in bufs], 2))
+        a = [w.copy() for w in ref]
+        ck(c.L.lh_upload_state(c.h, *[_dp(b) for b in a]))
+        nu = [np.ones(2 * s.ncols * n) for n in (s.nyu, s.nyv, s.nyu)]
+        ck(c.L.lh_download_nu(c.h, *[_dp(b) for b in nu]))
+        assert not any(x.any() for x in nu)
+        c.step(2)
+        ck(c.L.lh_download_state(c.h, *[_dp(b) for b in a]))
+        for k, (x, y) in enumerate(zip(a, bufs)):
+            assert np.array_equal(x, y), k
+    c.close()
