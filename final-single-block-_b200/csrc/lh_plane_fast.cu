@@ -122,68 +122,6 @@ __global__ void __launch_bounds__(LH_ZINV_T, LH_MINB(NZ, LH_ZINV_B)) k_zinv_f(co
 }
 
 // ---------------------------------------------------------------------------
-// The same z inverse with the threads of a vector in one warp (vector-major:
-// thread t works on x mode t / VT, VT = max(N1, N2) in {8, 16}), so the
-// exchange between the two passes is warp-local: a __syncwarp instead of
-// block barriers, and the warps of a CTA never wait on one another.  The
-// N1 x N2 exchange matrix of a vector is stored with a padded row (N2 + 1)
-// so the column-wise reads of the second pass are free of bank conflicts.
-// Same arithmetic as k_zinv_f, element for element.
-template <int NZ>
-__global__ void __launch_bounds__(LH_ZINV_T, LH_ZINV_B) k_zinv_w(const Inst *__restrict__ insts, const Work *__restrict__ work,
-                                                         int count, int cb)
-{
-    constexpr int N1 = Plan2<NZ>::N1, N2 = Plan2<NZ>::N2;
-    constexpr int VT = N1 > N2 ? N1 : N2;
-    // sizes whose vectors do not fit a warp are never launched (zinv_warp_size)
-    if constexpr (32 % VT != 0) return;
-    constexpr int LD = N2 + 1;
-    constexpr int Nz = 2 * NZ / 3;
-    extern __shared__ double2 sm[];
-    if ((int)blockIdx.x >= count) return;
-    const double2 *tw = insts[work[blockIdx.x].inst].twz;
-    const int t = threadIdx.x, v = t / VT, r = t % VT;
-    const double2 twr = __ldg(tw + (r < N2 ? r : 0));
-    const Work w = work[blockIdx.x];
-    const Inst &I = insts[w.inst];
-    const int nxh = I.nxh, nc = I.nc;
-    const int nblk = (nxh + cb - 1) / cb;
-    const int f = w.blk / nblk, i = (w.blk % nblk) * cb + v;
-    const bool ok = v < cb && i < nxh;
-    double2 *T = sm + (size_t)(v < cb ? v : 0) * N1 * LD;
-    const double2 *src = (f == 0 ? I.U1 : (f == 1 ? I.U3 : I.U2)) + (size_t)w.j * nc;
-    if (v < cb && r < N2) {
-        double2 a[N1];
-#pragma unroll
-        for (int n1 = 0; n1 < N1; n1++) {
-            const int n = r + N2 * n1;
-            int kr = -1;
-            if (n < Nz / 2) kr = n;
-            else if (n >= NZ - Nz / 2) kr = n - (NZ - Nz);
-            a[n1] = (kr >= 0 && ok) ? src[kr * nxh + i] : make_double2(0.0, 0.0);
-        }
-        DFT<N1, +1, NZ>::run(a, tw);
-        TwStep ts(twr);
-#pragma unroll
-        for (int k1 = 0; k1 < N1; k1++) {
-            double2 z = a[k1];
-            if (k1 > 0) z = twiddle<+1>(ts.next(), z);
-            T[k1 * LD + r] = z;
-        }
-    }
-    __syncwarp();
-    if (ok && r < N1) {
-        double2 b[N2];
-#pragma unroll
-        for (int n2 = 0; n2 < N2; n2++) b[n2] = T[r * LD + n2];
-        DFT<N2, +1, NZ>::run(b, tw);
-        double2 *dst = sin_field(I, w.slot, f) + i;
-#pragma unroll
-        for (int k2 = 0; k2 < N2; k2++) dst[(size_t)(r + N1 * k2) * nxh] = b[k2];
-    }
-}
-
-// ---------------------------------------------------------------------------
 // x transforms and products of one (plane j, block of rb z rows): xrow on rows
 // gathered from Sin with the y interpolations (interp_v FOU3D.f90:407, interp_u
 // :387): u1(j), u3(j); u2 at centre j, u2(j); u1, u3 at face j -> Sprod[slot]
@@ -353,106 +291,6 @@ __global__ void __launch_bounds__(LH_ZFWD_T, LH_MINB(NZ, LH_ZFWD_B)) k_zfwd_f(co
 }
 
 // ---------------------------------------------------------------------------
-// The same z forward with the threads of a vector in one warp.  Vector v is
-// (product f = v / cb, x mode c = v % cb), so the two vectors of a warp are
-// neighbouring x modes of one product and its loads of a z row share their
-// sectors.  Both transform passes are warp-local (__syncwarp); one block
-// barrier precedes the masks and derivatives, which combine the three
-// products of an x mode.  Each vector owns one region of max(NZ, N1 (N2+1))
-// complex (the padded exchange matrix, then the scaled spectrum in natural
-// order).  Same arithmetic as k_zfwd_f, element for element.
-template <int NZ>
-__global__ void __launch_bounds__(LH_ZFWD_T, LH_ZFWD_B) k_zfwd_w(const Inst *__restrict__ insts, const Work *__restrict__ work,
-                                                         int count, int cb)
-{
-    constexpr int N1 = Plan2<NZ>::N1, N2 = Plan2<NZ>::N2;
-    constexpr int VT = N1 > N2 ? N1 : N2;
-    if constexpr (32 % VT != 0) return;  // never launched (zfwd_warp_size)
-    constexpr int LD = N2 + 1;
-    // region stride rounded up to odd (in double2): the masks step reads the
-    // same z row of neighbouring modes' regions, which then fall in
-    // different banks
-    constexpr int REG = (NZ > N1 * LD ? NZ : N1 * LD) | 1;
-    constexpr int Nz = 2 * NZ / 3;
-    extern __shared__ double2 sm[];
-    if ((int)blockIdx.x >= count) return;
-    const double2 *tw = insts[work[blockIdx.x].inst].twz;
-    const int t = threadIdx.x, v = t / VT, r = t % VT;
-    const int f = v / cb, c = v % cb;
-    const bool live = f < 3;
-    const double2 twr = __ldg(tw + (r < N2 ? r : 0));
-    const Work w = work[blockIdx.x];
-    const Inst &I = insts[w.inst];
-    const int nxh = I.nxh, nc = I.nc, j = w.j;
-    const int h = w.blk & 1;
-    const int i0 = (w.blk >> 1) * cb, i = i0 + c;
-    const int g = h == 0 ? (f == 2 ? 3 : f) : (f == 0 ? 2 : f + 3);  // product of this vector
-    const double2 *S = sprod_slot(I, w.slot);
-    const bool ok = live && i < nxh;
-    double2 *z = sm + (size_t)(live ? v : 0) * REG;
-    {
-        double2 a[N1];
-        if (live && r < N2) {
-#pragma unroll
-            for (int n1 = 0; n1 < N1; n1++)
-                a[n1] = ok ? S[((size_t)g * NZ + r + N2 * n1) * nxh + i] : make_double2(0.0, 0.0);
-            DFT<N1, -1, NZ>::run(a, tw);
-            TwStep ts(twr);
-#pragma unroll
-            for (int k1 = 0; k1 < N1; k1++) {
-                double2 y = a[k1];
-                if (k1 > 0) y = twiddle<-1>(ts.next(), y);
-                z[k1 * LD + r] = y;
-            }
-        }
-    }
-    __syncwarp();
-    {
-        double2 b[N2];
-        if (live && r < N1) {
-#pragma unroll
-            for (int n2 = 0; n2 < N2; n2++) b[n2] = z[r * LD + n2];
-            DFT<N2, -1, NZ>::run(b, tw);
-        }
-        __syncwarp();
-        if (live && r < N1) {
-            const double dn1 = 1.0 / NZ;
-#pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) z[r + N1 * k2] = make_double2(dn1 * b[k2].x, dn1 * b[k2].y);
-        }
-    }
-    __syncthreads();
-    const FastDiv by_cb(cb);
-    for (int e = t; e < Nz * cb; e += blockDim.x) {
-        const int kr = by_cb.div(e), cc = by_cb.mod(e, kr), ii = i0 + cc;
-        if (ii >= nxh) continue;
-        const int zp = kr < Nz / 2 ? kr : kr + NZ - Nz;
-        const double2 p0 = sm[(size_t)cc * REG + zp], p1 = sm[(size_t)(cb + cc) * REG + zp],
-                      p2 = sm[(size_t)(2 * cb + cc) * REG + zp];
-        const size_t on = (size_t)(j - 1) * nc + kr * nxh + ii;
-        const bool keep = kr != Nz / 2;  // der_x/der_z zero the kz = -Nz/2 row (FOU3D.f90:444-447)
-        const double kx = I.kx[ii], kz = I.kz[kr];
-        if (h == 0) {  // p0 uu, p1 uw, p2 ww
-            double2 n1 = make_double2(0.0, 0.0), n3 = n1;
-            if (keep) {
-                n1 = add_ik(kz, p1, ik(kx, p0));
-                n3 = add_ik(kz, p2, ik(kx, p1));
-            }
-            I.NXZ1[on] = n1;
-            I.NXZ3[on] = n3;
-        } else {  // p0 vv, p1 uv, p2 wv
-            const size_t o = (size_t)j * nc + kr * nxh + ii;
-            I.VVC[o] = p0;
-            I.UVF[o] = p1;
-            I.WVF[o] = p2;
-            double2 n2 = make_double2(0.0, 0.0);
-            if (keep) n2 = add_ik(kz, p2, ik(kx, p1));
-            I.NXZ2[on] = n2;
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // host dispatch
 int fast_max_threads(int stage) { return stage == 0 ? LH_ZINV_T : LH_ZFWD_T; }
 
@@ -500,27 +338,6 @@ int fast_threads(int n, int vectors)
     return ((t + 31) / 32) * 32;
 }
 
-// z-inverse sizes whose vectors fit a warp (max(N1, N2) divides 32), and
-// whether the warp-local variant is selected (LH_ZINV_WARP=1).
-static bool zinv_warp_size(int n)
-{
-    switch (n) {
-#define LH_CASE(N) \
-    case N:        \
-        return 32 % (Plan2<N>::N1 > Plan2<N>::N2 ? Plan2<N>::N1 : Plan2<N>::N2) == 0;
-        LH_FAST_SIZES(LH_CASE)
-#undef LH_CASE
-    default:
-        return false;
-    }
-}
-
-static bool zinv_warp(int n)
-{
-    const char *ev = getenv("LH_ZINV_WARP");
-    return ev && ev[0] == '1' && zinv_warp_size(n);
-}
-
 // x stage: z rows per CTA for a bound rb (whole warps, at most kXprodThreads
 // lanes), its threads and shared memory
 int xprod_rows(int n, int rb)
@@ -556,50 +373,13 @@ size_t xprod_smem(int n, int rb)
     }
 }
 
-// z forward: sizes whose vectors fit a warp, the LH_ZFWD_WARP=1 selection,
-// threads and shared memory of a CTA of cb x modes (3 cb vectors)
-static bool zfwd_warp(int n)
-{
-    const char *ev = getenv("LH_ZFWD_WARP");
-    return ev && ev[0] == '1' && zinv_warp_size(n);
-}
+// Threads and shared memory of a z-forward CTA of cb x modes (3 cb vectors), shared
+// memory of a z-inverse CTA of cb vectors.
+int zfwd_threads(int n, int cb) { return fast_threads(n, 3 * cb); }
 
-int zfwd_threads(int n, int cb)
-{
-    if (!zfwd_warp(n)) return fast_threads(n, 3 * cb);
-    return ((3 * cb * fast_vector_threads(n) + 31) / 32) * 32;
-}
+size_t zfwd_smem(int n, int cb) { return (size_t)n * ((3 * cb) | 1) * sizeof(double2); }
 
-size_t zfwd_smem(int n, int cb)
-{
-    if (!zfwd_warp(n)) return (size_t)n * ((3 * cb) | 1) * sizeof(double2);
-    switch (n) {
-#define LH_CASE(N)                                                                                  \
-    case N: {                                                                                       \
-        const int reg = (N > Plan2<N>::N1 * (Plan2<N>::N2 + 1) ? N : Plan2<N>::N1 * (Plan2<N>::N2 + 1)) | 1; \
-        return (size_t)3 * cb * reg * sizeof(double2);                                            \
-    }
-        LH_FAST_SIZES(LH_CASE)
-#undef LH_CASE
-    default:
-        return 0;
-    }
-}
-
-// Shared memory of a z-inverse CTA of cb vectors.
-size_t zinv_smem(int n, int cb)
-{
-    if (!zinv_warp(n)) return (size_t)n * cb * sizeof(double2);
-    switch (n) {
-#define LH_CASE(N) \
-    case N:        \
-        return (size_t)cb * Plan2<N>::N1 * (Plan2<N>::N2 + 1) * sizeof(double2);
-        LH_FAST_SIZES(LH_CASE)
-#undef LH_CASE
-    default:
-        return 0;
-    }
-}
+size_t zinv_smem(int n, int cb) { return (size_t)n * cb * sizeof(double2); }
 
 cudaError_t fast_set_attributes(int Mz, int Mx, size_t smz, size_t smx, size_t smf)
 {
@@ -608,9 +388,7 @@ cudaError_t fast_set_attributes(int Mz, int Mx, size_t smz, size_t smx, size_t s
 #define LH_CASE(N)                                        \
     case N:                                               \
         e = raise_smem_limit((const void *)k_zinv_f<N>, smz); \
-        if (e == cudaSuccess) e = raise_smem_limit((const void *)k_zinv_w<N>, smz); \
         if (e == cudaSuccess) e = raise_smem_limit((const void *)k_zfwd_f<N>, smf); \
-        if (e == cudaSuccess) e = raise_smem_limit((const void *)k_zfwd_w<N>, smf); \
         break;
         LH_FAST_SIZES(LH_CASE)
 #undef LH_CASE
@@ -637,8 +415,7 @@ void fast_launch_zinv(int Mz, unsigned grid, int threads, size_t smem, cudaStrea
     switch (Mz) {
 #define LH_CASE(N)                                                                   \
     case N:                                                                          \
-        if (zinv_warp(N)) k_zinv_w<N><<<grid, threads, smem, st>>>(insts, work, count, cb); \
-        else k_zinv_f<N><<<grid, threads, smem, st>>>(insts, work, count, cb);       \
+        k_zinv_f<N><<<grid, threads, smem, st>>>(insts, work, count, cb);       \
         break;
         LH_FAST_SIZES(LH_CASE)
 #undef LH_CASE
@@ -664,8 +441,7 @@ void fast_launch_zfwd(int Mz, unsigned grid, int threads, size_t smem, cudaStrea
     switch (Mz) {
 #define LH_CASE(N)                                                                   \
     case N:                                                                          \
-        if (zfwd_warp(N)) k_zfwd_w<N><<<grid, threads, smem, st>>>(insts, work, count, cb); \
-        else k_zfwd_f<N><<<grid, threads, smem, st>>>(insts, work, count, cb);       \
+        k_zfwd_f<N><<<grid, threads, smem, st>>>(insts, work, count, cb);       \
         break;
         LH_FAST_SIZES(LH_CASE)
 #undef LH_CASE
