@@ -67,6 +67,15 @@ __device__ __forceinline__ double2 *sprod_slot(const Inst &I, int s)
 // ---------------------------------------------------------------------------
 // z inverse of one (y row jp, field f in {u1, u3, u2}, block of cb x modes):
 // the pruned cft of four_to_phys_u (FOU3D.f90:653-679), -> Sin[slot][f]
+// Elements from one k1 block of v vectors to the next in the exchange of a two-pass z
+// transform: the threads write it in their own order, and the second pass, whose
+// neighbouring rows are whole blocks apart, reads on from bank to bank as well.
+template <int NZ>
+__host__ __device__ constexpr int zblock(int v)
+{
+    return Plan2<NZ>::N2 * v + ((v * (1 + 7 * Plan2<NZ>::N2)) & 7);
+}
+
 template <int NZ>
 __global__ void __launch_bounds__(LH_ZINV_T, LH_MINB(NZ, LH_ZINV_B)) k_zinv_f(const Inst *__restrict__ insts, const Work *__restrict__ work,
                                                          int count, int cb)
@@ -77,7 +86,7 @@ __global__ void __launch_bounds__(LH_ZINV_T, LH_MINB(NZ, LH_ZINV_B)) k_zinv_f(co
     double2 *T = sm;
     if ((int)blockIdx.x >= count) return;
     const double2 *tw = insts[work[blockIdx.x].inst].twz;  // depends on Mz only
-    const int t = threadIdx.x, v = t % cb, r = t / cb;
+    const int t = threadIdx.x, v = t % cb, r = t / cb, zb = zblock<NZ>(cb);
     const double2 twr = __ldg(tw + r);  // outer-twiddle base W^r, issued before the data loads
     {
         const Work w = work[blockIdx.x];
@@ -103,14 +112,14 @@ __global__ void __launch_bounds__(LH_ZINV_T, LH_MINB(NZ, LH_ZINV_B)) k_zinv_f(co
             for (int k1 = 0; k1 < N1; k1++) {
                 double2 z = a[k1];
                 if (k1 > 0) z = twiddle<+1>(ts.next(), z);
-                T[(k1 * N2 + r) * cb + v] = z;
+                T[k1 * zb + t] = z;
             }
         }
         __syncthreads();
         if (r < N1) {
             double2 b[N2];
 #pragma unroll
-            for (int n2 = 0; n2 < N2; n2++) b[n2] = T[(r * N2 + n2) * cb + v];
+            for (int n2 = 0; n2 < N2; n2++) b[n2] = T[r * zb + n2 * cb + v];
             DFT<N2, +1, NZ>::run(b, tw);
             if (ok) {
                 double2 *dst = sin_field(I, w.slot, f) + i;
@@ -138,41 +147,44 @@ __global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 6 ? 4 : (XPlan
     k_xprod_r(const Inst *__restrict__ insts, const Work *__restrict__ work, int rb, int want_max)
 {
     using XP = XPlan<NX>;
+    using XK = XPack<NX>;
     constexpr int KQ = XP::KQ, nxh = NX / 3 + 1;
     extern __shared__ double2 sm[];
     const Work w = work[blockIdx.x];
     const Inst &I = insts[w.inst];
-    const int lane = threadIdx.x & 31, r = lane % XP::N1;
-    const bool on = lane < XP::RW * XP::N1;
-    const int row = (threadIdx.x >> 5) * XP::RW + (on ? lane / XP::N1 : 0);
     const int Mz = I.Mz, j = w.j;
-    const int q = w.blk * rb + row;  // this lane's z row
-    const bool rowok = on && row < rb && q < Mz;
-    // this row in the planes the y interpolations read
-    const size_t fs = (size_t)Mz * nxh, orow = (size_t)min(q, Mz - 1) * nxh;
-    const double2 *u1j = sin_field(I, w.aux + 1, 0) + orow, *u3j = u1j + fs, *vj = u3j + fs;
-    const double2 *vjm = sin_field(I, w.aux, 2) + orow;
-    const double2 *u1p = sin_field(I, w.aux + 2, 0) + orow, *u3p = u1p + fs;
-    double2 *S = sprod_slot(I, w.slot) + orow;
+    // first z row of this warp and how many there are; not packed: this lane's row and
+    // whether there is one
+    const int lane = threadIdx.x & 31;
+    const bool on = lane < XP::RW * XP::N1;
+    const int row0 = (threadIdx.x >> 5) * XP::RW + (XK::value || !on ? 0 : lane / XP::N1), q0 = w.blk * rb + row0;
+    const int left = min(rb - row0, Mz - q0), rows = XK::value ? min(XP::RW, left) : (on && left > 0);
+    // this row in the planes the y interpolations read, in field strides from u1(j): u2(j-1)
+    // -1, u1(j) 0, u3(j) 1, u2(j) 2, u1(j+1) 3, u3(j+1) 4; 32-bit offsets
+    const int fs = Mz * nxh;
+    const double2 *const U = sin_field(I, w.aux + 1, 0) + (size_t)min(q0, Mz - 1) * nxh;
+    double2 *const S = sprod_slot(I, w.slot) + (size_t)min(q0, Mz - 1) * nxh;
     const double dnv = 1.0 / (I.yv[j] - I.yv[j - 1]), dnu = 1.0 / (I.yu[j + 1] - I.yu[j]);
     const double w0v = (I.yu[j] - I.yv[j - 1]) * dnv, w1v = (I.yv[j] - I.yu[j]) * dnv;
     const double w0u = (I.yv[j] - I.yu[j]) * dnu, w1u = (I.yu[j + 1] - I.yv[j]) * dnu;
     const bool track = want_max && I.dt_mode == 0 && j <= I.nyu - 1;  // maxima over planes 1..nyu-1
     double m1 = 0.0, m3 = 0.0;
-    xrow<NX>(
-        sm + (size_t)row * XP::N1 * XP::LD, I.twx, r, on, rowok, track, m1, m3,
-        [&](int pair, const int *k, double2 *A, double2 *B) {
+    xrow<NX, XK::value>(
+        sm + (size_t)row0 * XK::RS, I.twx, rows, track, m1, m3,
+        [&](int pair, int row, const int *k, double2 *A, double2 *B) {
+            const int o = row * nxh;
+            auto ld = [&](int q, int n1) { return U[q * fs + o + k[n1]]; };
             if (pair == 0) {  // (u1, u3) at the centre
 #pragma unroll
                 for (int n1 = 0; n1 < KQ; n1++) {
-                    A[n1] = u1j[k[n1]];
-                    B[n1] = u3j[k[n1]];
+                    A[n1] = ld(0, n1);
+                    B[n1] = ld(1, n1);
                 }
             } else if (pair == 1) {  // u2 at the centre and at the face
 #pragma unroll
                 for (int n1 = 0; n1 < KQ; n1++) {
-                    A[n1] = vjm[k[n1]];
-                    B[n1] = vj[k[n1]];
+                    A[n1] = ld(-1, n1);
+                    B[n1] = ld(2, n1);
                 }
 #pragma unroll
                 for (int n1 = 0; n1 < KQ; n1++)
@@ -181,10 +193,10 @@ __global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 6 ? 4 : (XPlan
                 double2 a1[KQ], b1[KQ];
 #pragma unroll
                 for (int n1 = 0; n1 < KQ; n1++) {
-                    A[n1] = u1p[k[n1]];
-                    a1[n1] = u1j[k[n1]];
-                    B[n1] = u3p[k[n1]];
-                    b1[n1] = u3j[k[n1]];
+                    A[n1] = ld(3, n1);
+                    a1[n1] = ld(0, n1);
+                    B[n1] = ld(4, n1);
+                    b1[n1] = ld(1, n1);
                 }
 #pragma unroll
                 for (int n1 = 0; n1 < KQ; n1++) {
@@ -193,9 +205,10 @@ __global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 6 ? 4 : (XPlan
                 }
             }
         },
-        [&](int pair, int k, double2 A, double2 B) {
-            S[(size_t)(2 * pair) * fs + k] = A;
-            S[(size_t)(2 * pair + 1) * fs + k] = B;
+        [&](int pair, int row, int k, double2 A, double2 B) {
+            const int o = 2 * pair * fs + row * nxh + k;
+            S[o] = A;
+            S[o + fs] = B;
         });
     if (track) xmax(I, m1, m3);
 }
@@ -216,8 +229,7 @@ __global__ void __launch_bounds__(LH_ZFWD_T, LH_MINB(NZ, LH_ZFWD_B)) k_zfwd_f(co
     double2 *T = sm;
     if ((int)blockIdx.x >= count) return;
     const double2 *tw = insts[work[blockIdx.x].inst].twz;  // depends on Mz only
-    // T[z][v] with an odd row stride ld (double2), as in the x stage
-    const int t = threadIdx.x, nv = 3 * cb, ld = nv | 1, v = t % nv, r = t / nv;
+    const int t = threadIdx.x, nv = 3 * cb, v = t % nv, r = t / nv, zb = zblock<NZ>(nv);
     const double2 twr = __ldg(tw + r);  // outer-twiddle base W^r, issued before the data loads
     const int f = v / cb, c = v % cb;
     const FastDiv by_cb(cb);
@@ -241,7 +253,7 @@ __global__ void __launch_bounds__(LH_ZFWD_T, LH_MINB(NZ, LH_ZFWD_B)) k_zfwd_f(co
             for (int k1 = 0; k1 < N1; k1++) {
                 double2 z = a[k1];
                 if (k1 > 0) z = twiddle<-1>(ts.next(), z);
-                T[(k1 * N2 + r) * ld + v] = z;
+                T[k1 * zb + t] = z;
             }
         }
         __syncthreads();
@@ -249,14 +261,14 @@ __global__ void __launch_bounds__(LH_ZFWD_T, LH_MINB(NZ, LH_ZFWD_B)) k_zfwd_f(co
             double2 b[N2];
             if (r < N1) {
 #pragma unroll
-                for (int n2 = 0; n2 < N2; n2++) b[n2] = T[(r * N2 + n2) * ld + v];
+                for (int n2 = 0; n2 < N2; n2++) b[n2] = T[r * zb + n2 * nv + v];
                 DFT<N2, -1, NZ>::run(b, tw);
             }
             __syncthreads();
             if (r < N1) {
                 const double dn1 = 1.0 / NZ;
 #pragma unroll
-                for (int k2 = 0; k2 < N2; k2++) T[(r + N1 * k2) * ld + v] = make_double2(dn1 * b[k2].x, dn1 * b[k2].y);
+                for (int k2 = 0; k2 < N2; k2++) T[(r + N1 * k2) * nv + v] = make_double2(dn1 * b[k2].x, dn1 * b[k2].y);
             }
         }
         __syncthreads();
@@ -264,7 +276,7 @@ __global__ void __launch_bounds__(LH_ZFWD_T, LH_MINB(NZ, LH_ZFWD_B)) k_zfwd_f(co
             const int kr = by_cb.div(e), cc = by_cb.mod(e, kr), ii = i0 + cc;
             if (ii >= nxh) continue;
             const int zp = kr < Nz / 2 ? kr : kr + NZ - Nz;
-            const double2 *row = T + zp * ld + cc;
+            const double2 *row = T + zp * nv + cc;
             const double2 p0 = row[0], p1 = row[cb], p2 = row[2 * cb];
             const size_t on = (size_t)(j - 1) * nc + kr * nxh + ii;
             const bool keep = kr != Nz / 2;  // der_x/der_z zero the kz = -Nz/2 row (FOU3D.f90:444-447)
@@ -366,7 +378,7 @@ size_t xprod_smem(int n, int rb)
 {
     switch (n) {
 #define LH_CASE(N) \
-    case N: return (size_t)rb * XPlan<N>::N1 * XPlan<N>::LD * sizeof(double2);
+    case N: return (size_t)rb * XPack<N>::RS * sizeof(double2);
         LH_FAST_SIZES(LH_CASE)
 #undef LH_CASE
     default: return 0;
@@ -377,9 +389,20 @@ size_t xprod_smem(int n, int rb)
 // memory of a z-inverse CTA of cb vectors.
 int zfwd_threads(int n, int cb) { return fast_threads(n, 3 * cb); }
 
-size_t zfwd_smem(int n, int cb) { return (size_t)n * ((3 * cb) | 1) * sizeof(double2); }
+static size_t exchange_smem(int n, int v)
+{
+    switch (n) {
+#define LH_CASE(N) \
+    case N: return (size_t)Plan2<N>::N1 * zblock<N>(v) * sizeof(double2);
+        LH_FAST_SIZES(LH_CASE)
+#undef LH_CASE
+    default: return 0;
+    }
+}
 
-size_t zinv_smem(int n, int cb) { return (size_t)n * cb * sizeof(double2); }
+size_t zfwd_smem(int n, int cb) { return exchange_smem(n, 3 * cb); }
+
+size_t zinv_smem(int n, int cb) { return exchange_smem(n, cb); }
 
 cudaError_t fast_set_attributes(int Mz, int Mx, size_t smz, size_t smx, size_t smf)
 {

@@ -40,7 +40,7 @@ struct SmallPlane {
     static constexpr size_t bytes = (plane + (size_t)G * XPlan<NX>::N1 * XPlan<NX>::LD) * sizeof(double2);
     static_assert(Z2 % 3 == 0 && Z2 <= Z1, "whole k2 rows are kept, every task has its lane");
     static_assert(Z1 == Plan2<NZ>::N1, "the staged kernels' split");
-    static_assert(XPlan<NX>::ROUNDS == 1, "a lane reads and writes the modes of one task");
+    static_assert(XPlan<NX>::N2 <= XPlan<NX>::N1, "a lane reads and writes the modes of one task");
 };
 
 template <int NX, int NZ>
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_plane_small(const Inst *__
     // ---- x transforms and products, row by row ----------------------------------
     {
         using XP = XPlan<NX>;
-        const int r = t % XP::N1, g = t / XP::N1;
+        const int g = t / XP::N1;
         double2 *const T = sm + SP::plane + (size_t)g * XP::N1 * XP::LD;
         const bool track = want_max && I.dt_mode == 0 && j <= I.nyu - 1;
         const double dnv = 1.0 / (I.yv[j] - I.yv[j - 1]), dnu = 1.0 / (I.yu[j + 1] - I.yu[j]);
@@ -119,9 +119,9 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_plane_small(const Inst *__
             const bool rowok = z < NZ;
             double2 *const row = P + (rowok ? z : 0) * LDX;
             double2 FA[XP::KQ], FB[XP::KQ];  // (u1, u3) at the face, interpolated before pair 0's products take its slots
-            xrow<NX>(
-                T, I.twx, r, true, rowok, track, m1, m3,
-                [&](int pair, const int *k, double2 *A, double2 *B) {
+            xrow<NX, false>(
+                T, I.twx, rowok, track, m1, m3,
+                [&](int pair, int, const int *k, double2 *A, double2 *B) {
                     if (pair == 0) {
 #pragma unroll
                         for (int n1 = 0; n1 < XP::KQ; n1++) {
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_plane_small(const Inst *__
                         for (int n1 = 0; n1 < XP::KQ; n1++) A[n1] = FA[n1], B[n1] = FB[n1];
                     }
                 },
-                [&](int pair, int k, double2 A, double2 B) {
+                [&](int pair, int, int k, double2 A, double2 B) {
                     row[2 * pair * FS + k] = A;
                     row[(2 * pair + 1) * FS + k] = B;
                 });

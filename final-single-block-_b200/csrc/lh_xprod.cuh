@@ -55,11 +55,14 @@ struct TwStep {
 //
 // A vector crosses shared memory twice (the exchanges, 4 accesses an element)
 // instead of 12 accesses when the gather, the products and the split went
-// through it too, which kept that pipe busier than the FP64 pipe.  Tasks come in
-// rounds of N1 whose sets are closed under m -> N2 - m, and a lane keeps its
-// columns of the matrix from one use to the next, so two __syncwarp a vector are
-// all the synchronisation.  Every load of a task is issued before the first is
-// used: loaded mode by mode the stage waited on L2 for half its time.
+// through it too.  That pipe is still the busiest (57 % of its cycles at Mx = 192,
+// against the FP64 pipe's 50 %), so the tasks of as many whole rows as fit sit on
+// consecutive lanes (24 of 32 at N2 = 12; spread over the rows' own lanes they
+// touched a quarter of a wavefront more), m -> N2 - m stays inside the row, and the
+// matrices of neighbouring rows are a task's columns apart in the banks.  A lane
+// keeps its columns of the matrix from one use to the next, so two __syncwarp a
+// vector are all the synchronisation.  Every load of a task is issued before the
+// first is used: loaded mode by mode the stage waited on L2 for half its time.
 template <int NX>
 struct XPlan {
     // the substep at the other splits, us: 192 as 8 x 24 394 (16 x 12: 362), 144 as
@@ -72,67 +75,98 @@ struct XPlan {
     static constexpr int N2 = NX / N1;
     static constexpr int LD = N2 | 1;             // odd row stride: conflict-free rows and columns
     static constexpr int KQ = NX / 3 / N2 + 1;    // modes k <= Nx/2 of a task, at most
-    static constexpr int ROUNDS = N2 <= N1 ? 1 : ((N2 + 1) / 2 + N1 / 2 - 1) / (N1 / 2);
     static constexpr int RW = 32 / N1;            // rows per warp; N1 = 6 and 12 leave lanes over
     static constexpr bool WHOLE = RW * N1 == 32;
     static_assert(N1 * N2 == NX && N1 % 2 == 0 && 2 * KQ <= N1 + 1, "modes, mirror images, zeros between");
 };
-// Task of lane r in round g and the lane that holds task N2 - m; -1: idle.
-// Round 0: m = 0 .. N1/2 - 1, N2/2, and the mirror images N2 - m downwards from
-// the last lane; round g: m = N1/2 g + .. and its mirror images.
-template <int N1, int N2>
-__device__ __forceinline__ void xtask(int g, int r, int &m, int &partner)
-{
-    constexpr int H = N1 / 2;
-    if (N2 <= N1) {
-        m = r < N2 ? r : -1;
-        partner = r < N2 ? (N2 - r) % N2 : r;
-    } else if (g == 0) {
-        m = r < H ? r : (r > H ? N2 - (N1 - r) : (N2 % 2 ? -1 : N2 / 2));
-        partner = (N1 - r) % N1;
-    } else {
-        partner = N1 - 1 - r;
-        const int a = H * g + (r < H ? r : partner);
-        m = 2 * a < N2 ? (r < H ? a : N2 - a) : -1;
+// Whether the tasks of RPR whole rows are packed on a warp's consecutive lanes or
+// every row's stay on its own N1 lanes: packed where they do not fit those, or touch
+// fewer groups of eight lanes (a quarter of an access's wavefronts each) that way.
+template <int NX>
+struct XPack {
+    using XP = XPlan<NX>;
+    static constexpr int N1 = XP::N1, N2 = XP::N2, RW = XP::RW;
+    static constexpr int groups()
+    {
+        int n = 0;
+        for (int g = 0; g < 4; g++)
+            for (int l = 8 * g; l < 8 * g + 8; l++)
+                if (l < RW * N1 && l % N1 < N2) {
+                    n++;
+                    break;
+                }
+        return n;
     }
-}
+    static constexpr bool value = N2 > N1 || (RW * N2 + 7) / 8 < groups();
+    static constexpr int RPR = 32 / N2 < RW ? 32 / N2 : RW;
+    // elements from one row's matrix to the next: in the banks the tasks of
+    // neighbouring rows follow one another (the lanes of the middle pass do where
+    // those cannot)
+    static constexpr int RS = N1 * XP::LD + (value ? ((RPR > 1 && (N1 % 8 == 0 || N1 >= N2) ? N2 : N1 * XP::LD) - N1 * XP::LD) & 7 : 0);
+};
 
-// The three pairs of a row: load(pair, k, A, B) fetches the modes k[] of the two
-// real rows, store(pair, k, A, B) takes the spectra of the two products at mode k.
-// T: the row's exchange matrix; r: this lane of the row's N1; m1, m3 gather max
-// |u1|, |u3| when track.  Every lane of the warp calls it, with rowok = false
-// past the rows and on = false on the lanes left over.
-template <int NX, class Load, class Store>
-__device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int r, bool on, bool rowok, bool track, double &m1,
-                                     double &m3, Load &&load, Store &&store)
+// The three pairs of a warp's RW rows: load(pair, row, k, A, B) fetches the modes k[]
+// of the two real rows, store(pair, row, k, A, B) takes the spectra of the two
+// products at mode k.  PACKED: T the warp's exchange matrices, RS apart, rows how many
+// of the rows there are.  Otherwise T is the matrix of this lane's row, rows whether
+// it exists, and row always 0.  m1, m3 gather max |u1|, |u3| when track.  Every lane
+// of the warp calls it.
+template <int NX, bool PACKED, class Load, class Store>
+__device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int rows, bool track, double &m1, double &m3,
+                                     Load &&load, Store &&store)
 {
     using XP = XPlan<NX>;
     constexpr int N1 = XP::N1, N2 = XP::N2, LD = XP::LD, KQ = XP::KQ, nxh = NX / 3 + 1;
-    const int group = (threadIdx.x & 31) - r;
+    constexpr int RW = XP::RW, RPR = PACKED ? XPack<NX>::RPR : RW, RS = XPack<NX>::RS, ROUNDS = (RW + RPR - 1) / RPR;
+    static_assert(PACKED || N2 <= N1, "a lane for every task");
+    const int lane = threadIdx.x & 31, r = lane % N1, lane_row = lane / N2, lane_task = lane - lane_row * N2;
+    const bool on = XP::WHOLE || lane < RW * N1;
+    double2 *const Tr = T + ((PACKED && on ? lane / N1 * RS : 0) + r * LD);  // row r of the matrix, the middle pass
+    // task m of `row`, the lane of task N2 - m.  What follows from packed ones is formed
+    // again in each round: kept for all three pairs it would spill.
+    struct Task {
+        int m, partner, row;
+        bool on, ok;
+        __device__ Task(int g, int tl, int tm, int r, bool lane_on, int rows) : m(tm), row(0)
+        {
+            if (PACKED) {
+                asm volatile("" : "+r"(tl), "+r"(m));
+                partner = tl * N2 + (m > 0 ? N2 - m : 0);
+                row = g * RPR + tl;
+                on = tl < RPR && (RW % RPR == 0 || row < RW);
+                ok = on && row < rows;
+            } else {
+                m = r < N2 ? r : -1;
+                partner = (int)(threadIdx.x & 31) - r + (r < N2 ? (N2 - r) % N2 : r);
+                on = m >= 0 && lane_on;
+                ok = on && rows != 0;
+            }
+        }
+    };
     double saved[N2];
 #pragma unroll 1
     for (int pair = 0; pair < 3; pair++) {
         // gather and inverse pass 1
 #pragma unroll 1
-        for (int g = 0; g < XP::ROUNDS; g++) {
-            int n2, partner;
-            xtask<N1, N2>(g, r, n2, partner);
+        for (int g = 0; g < ROUNDS; g++) {
+            const Task q(g, lane_row, lane_task, r, on, rows);
+            double2 *const Tm = T + (q.row * RS + q.m);
             double2 a[N1], mir[KQ], A[KQ], B[KQ];
             // every load of the task before the first use (indices past the
             // modes are clamped, their values dropped)
             int kk[KQ];
 #pragma unroll
             for (int n1 = 0; n1 < KQ; n1++) {
-                const int k = (n2 >= 0 ? n2 : 0) + N2 * n1;
+                const int k = (q.m >= 0 ? q.m : 0) + N2 * n1;
                 kk[n1] = k < nxh ? k : 0;
             }
-            load(pair, kk, A, B);
+            load(pair, q.ok ? q.row : 0, kk, A, B);
 #pragma unroll
             for (int k1 = 0; k1 < N1; k1++) a[k1] = make_double2(0.0, 0.0);
 #pragma unroll
             for (int n1 = 0; n1 < KQ; n1++) {
-                const int k = n2 + N2 * n1;
-                const bool in = rowok && n2 >= 0 && k < nxh;
+                const int k = q.m + N2 * n1;
+                const bool in = q.ok && k < nxh;
                 if (!in) A[n1] = B[n1] = make_double2(0.0, 0.0);
                 if (k == 0) A[n1].y = B[n1].y = 0.0;  // Im of mode 0 dropped (rft_buff.f:78-81)
                 a[n1] = make_double2(A[n1].x - B[n1].y, A[n1].y + B[n1].x);
@@ -140,25 +174,25 @@ __device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int r, bool 
             }
 #pragma unroll
             for (int n1 = 0; n1 < KQ; n1++) {
-                const double2 z = make_double2(__shfl_sync(0xffffffffu, mir[n1].x, group + partner),
-                                               __shfl_sync(0xffffffffu, mir[n1].y, group + partner));
+                const double2 z = make_double2(__shfl_sync(0xffffffffu, mir[n1].x, q.partner),
+                                               __shfl_sync(0xffffffffu, mir[n1].y, q.partner));
                 // z[NX - k] sits at N1 - 1 - n1 on the partner; task 0 is its own, one higher
                 const double2 own = n1 + 1 < KQ ? mir[n1 + 1] : make_double2(0.0, 0.0);
-                a[N1 - 1 - n1] = n2 == 0 ? own : z;
+                a[N1 - 1 - n1] = q.m == 0 ? own : z;
             }
             DFT<N1, +1, NX>::run(a, tw);
-            if (n2 >= 0 && (XP::WHOLE || on)) {
-                TwStep ts(__ldg(tw + n2));
+            if (q.on) {
+                TwStep ts(__ldg(tw + q.m));
 #pragma unroll
-                for (int k1 = 0; k1 < N1; k1++) T[k1 * LD + n2] = k1 > 0 ? twiddle<+1>(ts.next(), a[k1]) : a[k1];
+                for (int k1 = 0; k1 < N1; k1++) Tm[k1 * LD] = k1 > 0 ? twiddle<+1>(ts.next(), a[k1]) : a[k1];
             }
         }
         __syncwarp();
-        // inverse pass 2, products, forward pass 1 of lane r's row of the matrix
+        // inverse pass 2, products, forward pass 1 of this lane's row of the matrix
         {
             double2 b[N2];
 #pragma unroll
-            for (int n2 = 0; n2 < N2; n2++) b[n2] = T[r * LD + n2];
+            for (int n2 = 0; n2 < N2; n2++) b[n2] = Tr[n2];
             DFT<N2, +1, NX>::run(b, tw);
             if (pair == 0) {
 #pragma unroll
@@ -185,33 +219,35 @@ __device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int r, bool 
             DFT<N2, -1, NX>::run(b, tw);
             TwStep ts(__ldg(tw + r));
 #pragma unroll
-            for (int m = 0; m < N2; m++) {
-                const double2 z = m > 0 ? twiddle<-1>(ts.next(), b[m]) : b[m];
-                if (XP::WHOLE || on) T[r * LD + m] = z;
+            for (int n2 = 0; n2 < N2; n2++) {
+                const double2 z = n2 > 0 ? twiddle<-1>(ts.next(), b[n2]) : b[n2];
+                if (on) Tr[n2] = z;
             }
         }
         __syncwarp();
         // forward pass 2, split, scale 1/Mx
 #pragma unroll 1
-        for (int g = 0; g < XP::ROUNDS; g++) {
-            int m, partner;
-            xtask<N1, N2>(g, r, m, partner);
+        for (int g = 0; g < ROUNDS; g++) {
+            const Task q(g, lane_row, lane_task, r, on, rows);
+            const int m = q.m;
+            // packed lanes without a task read nothing, others their row's first column
+            const double2 *const Tm = T + (q.row * RS + (m >= 0 ? m : 0));
             double2 e[N1];
 #pragma unroll
-            for (int k1 = 0; k1 < N1; k1++) e[k1] = T[k1 * LD + (m >= 0 ? m : 0)];
+            for (int k1 = 0; k1 < N1; k1++) e[k1] = !PACKED || q.on ? Tm[k1 * LD] : make_double2(0.0, 0.0);
             DFT<N1, -1, NX>::run(e, tw);
             const double h = 0.5 / NX;
 #pragma unroll
             for (int k1 = 0; k1 < KQ; k1++) {
-                const double2 z = make_double2(__shfl_sync(0xffffffffu, e[N1 - 1 - k1].x, group + partner),
-                                               __shfl_sync(0xffffffffu, e[N1 - 1 - k1].y, group + partner));
+                const double2 z = make_double2(__shfl_sync(0xffffffffu, e[N1 - 1 - k1].x, q.partner),
+                                               __shfl_sync(0xffffffffu, e[N1 - 1 - k1].y, q.partner));
                 const int k = m + N2 * k1;
                 const double2 zk = e[k1], own = e[(N1 - k1) % N1], zm = m == 0 ? own : z;
-                if (rowok && m >= 0 && k < nxh) {
+                if (q.ok && k < nxh) {
                     double2 A = make_double2(h * (zk.x + zm.x), h * (zk.y - zm.y));
                     double2 B = make_double2(h * (zk.y + zm.y), h * (zm.x - zk.x));
                     if (k == 0) A.y = B.y = 0.0;
-                    store(pair, k, A, B);
+                    store(pair, q.row, k, A, B);
                 }
             }
         }
