@@ -3,6 +3,8 @@
 #include "lh_engine.h"
 
 #include <cuda.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cstdint>
@@ -308,6 +310,30 @@ static cudaError_t upload_fields(DevInstance &d, const double *const *src, doubl
     return e;
 }
 
+// Page faults of a pageable buffer that a copy is about to fill, in one call: one by
+// one inside the copy they cost more than the copy itself (lh_download_state into
+// fresh memory, 26 MB 12.6 -> 8.1 ms, 82 MB 40 -> 25 ms).  Whole pages inside the buffer
+// only; left to the copy where four pages across the buffer are there already
+// (walking those takes a tenth of their copy) and where the kernel lacks the call.
+void prefault(void *p, size_t bytes)
+{
+#ifdef MADV_POPULATE_WRITE
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t a = ((uintptr_t)p + page - 1) / page * page, b = ((uintptr_t)p + bytes) / page * page;
+    if (b <= a || b - a < 16 * page) return;
+    bool there = true;
+    for (int k = 0; k < 4 && there; k++) {
+        unsigned char v = 0;
+        const uintptr_t q = a + (b - a - page) / page * k / 3 * page;
+        there = mincore((void *)q, page, &v) == 0 && (v & 1);
+    }
+    if (there) return;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) cudaGetLastError();
+    else if (at.type == cudaMemoryTypeUnregistered) madvise((void *)a, b - a, MADV_POPULATE_WRITE);
+#endif
+}
+
 cudaError_t download_field(const DevInstance &d, const double2 *src, int len, double *dst, cudaStream_t st)
 {
     FieldSet f;
@@ -317,7 +343,9 @@ cudaError_t download_field(const DevInstance &d, const double2 *src, int len, do
     f.len[0] = len;
     cudaError_t e = planes_to_cols(f, 1, st);
     if (e != cudaSuccess) return e;
-    return cudaMemcpyAsync(dst, d.stage, (size_t)len * f.nc * sizeof(double2), cudaMemcpyDeviceToHost, st);
+    const size_t bytes = (size_t)len * f.nc * sizeof(double2);
+    prefault(dst, bytes);
+    return cudaMemcpyAsync(dst, d.stage, bytes, cudaMemcpyDeviceToHost, st);
 }
 
 // The Nu reset and the scalars of an upload (getini).

@@ -56,6 +56,8 @@ cudaError_t instance_upload(DevInstance &d, const double *u1, const double *u2, 
 cudaError_t instance_upload_p_last(DevInstance &d, const double *u1, const double *u2, const double *u3,
                                    const double *p, cudaStream_t st, cudaEvent_t ev_u);
 cudaError_t instance_download(DevInstance &d, double *u1, double *u2, double *u3, double *p, cudaStream_t st);
+// take a pageable buffer's page faults before a copy fills it
+void prefault(void *p, size_t bytes);
 cudaError_t download_field(const DevInstance &d, const double2 *src, int len, double *dst, cudaStream_t st);
 
 // Device resources of the diagnostics (lh_diag.cu): the pressure snapshot the

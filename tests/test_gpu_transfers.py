@@ -78,3 +78,42 @@ def test_transfers(N, kind):
         for k, (x, y) in enumerate(zip(a, bufs)):
             assert np.array_equal(x, y), k
     c.close()
+
+
+@pytest.mark.parametrize("N", [(16, 16, 33), (48, 32, 65), (64, 64, 130)])
+def test_pageable_downloads(N):
+    """Spectra and state into fresh pageable memory (large ones in page-locked pieces, the
+    last not whole; pages taken beforehand) equal those into page-locked memory."""
+    import ctypes
+    import mmap
+
+    import torch
+    from lh_b200 import Desc, Engine
+    from lh_b200.capi import _dp
+    e = Engine(Desc(Nx=N[0], Nz=N[1], ny=N[2], dt_mode=1, dt=1e-4))
+    s = e.sizes
+    rng = np.random.default_rng(5)
+    e.upload(*[1e-3 * (rng.standard_normal((s.ncols, n)) + 1j * rng.standard_normal((s.ncols, n)))
+               for n in (s.nyu + 2, s.nyv + 2, s.nyu + 2, s.nyu)])
+    for _ in range(3):
+        e.spectra_accumulate()
+
+    def fresh(n):
+        return np.frombuffer(mmap.mmap(-1, 8 * n + 24), dtype=np.float64)[1:n + 1]
+
+    def spectra(w, n, a):
+        assert e.L.lh_get_spectra(e.h, w, _dp(a), n, ctypes.byref(ctypes.c_int())) == n
+        return a
+
+    for w in range(5):
+        n = e.L.lh_get_spectra(e.h, w, None, 0, None)
+        want = spectra(w, n, torch.zeros(n, dtype=torch.float64).pin_memory().numpy())
+        assert want.any()
+        a = fresh(n)
+        assert np.array_equal(spectra(w, n, a), want) and np.array_equal(spectra(w, n, a), want)
+    sizes = [2 * s.ncols * n for n in (s.nyu + 2, s.nyv + 2, s.nyu + 2, s.nyu)]
+    got = [[torch.zeros(n, dtype=torch.float64).pin_memory().numpy() for n in sizes], [fresh(n) for n in sizes]]
+    for b in got:
+        assert e.L.lh_download_state(e.h, *[_dp(x) for x in b]) == 0
+    assert all(np.array_equal(x, y) for x, y in zip(*got))
+    e.close()
