@@ -61,7 +61,13 @@ extern "C" int lh_ctx_create(const lh_grid_desc *desc, lh_ctx **out)
         return LH_ECUDA;
     }
     const HostSetup &s = c->dev.hs;
-    Tiles t = default_tiles(s.Mx, s.Mz, s.nxh, s.nyu);
+    // the larger staging of a lone instance where the device has room to spare
+    Tiles t = default_tiles(s.Mx, s.Mz, s.nxh, s.nyu, true);
+    size_t room = 0, total = 0;
+    if (cudaMemGetInfo(&room, &total) != cudaSuccess || room / 2 < instance_bytes(s, t.chunk)) {
+        cudaGetLastError();
+        t = default_tiles(s.Mx, s.Mz, s.nxh, s.nyu);
+    }
     const char *gen = getenv("LH_GENERIC_FFT");
     e = instance_alloc(c->dev, t.chunk, c->st);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_inst, sizeof(Inst));

@@ -37,14 +37,19 @@ size_t staging_units(int chunk) { return (size_t)(chunk + 2 * kRoundStreams) * 3
 
 // Bytes of plane staging one chunk round may use across all instances of a
 // plan, kept well inside the 126 MB L2 (LH_STAGING_MB overrides, for tuning).
-size_t staging_budget()
+// A lone instance takes 300 MB: its rounds' staging then spills to HBM, which the
+// plane pass leaves mostly idle, but fewer launches, each of several full waves, are
+// worth more.  Substep on B200, us, 96 / 150 / 200 / 300 / 500 MB: 128x128x153 357 354
+// 355 351 352, 192x192x257 1502 1478 1467 1452 1442, 256x256x257 2642 2629 2616 2613
+// 2604, 216x216x129 1026 975 971 971 969; an odd number of rounds loses up to 5 %.
+size_t staging_budget(bool lone)
 {
     const char *ev = getenv("LH_STAGING_MB");
     const long mb = ev ? atol(ev) : 0;
-    return (size_t)(mb > 0 ? mb : 96) << 20;
+    return (size_t)(mb > 0 ? mb : lone ? 300 : 96) << 20;
 }
 
-Tiles default_tiles(int Mx, int Mz, int nxh, int nyu)
+Tiles default_tiles(int Mx, int Mz, int nxh, int nyu, bool lone)
 {
     Tiles t;
     const size_t target = 48 * 1024;
@@ -55,7 +60,7 @@ Tiles default_tiles(int Mx, int Mz, int nxh, int nyu)
     // staging capacity: the fast path holds 9 plane fields per plane plus 6
     // for the halo rows (staging_units), the generic path 6 per plane
     const size_t unit = (size_t)Mz * nxh * sizeof(double2);
-    const size_t units = staging_budget() / unit;
+    const size_t units = staging_budget(lone) / unit;
     const size_t fixed = 6 * kRoundStreams;
     t.chunk = (int)std::max<size_t>(kRoundStreams, std::min<size_t>((size_t)nyu + kRoundStreams - 1,
                                                                   units > fixed ? (units - fixed) / 9 : kRoundStreams));
@@ -534,7 +539,7 @@ TuneParams default_params(const HostSetup &s)
 {
     TuneParams t;
     if (fast_size(s.Mz) && fast_size(s.Mx)) default_bounds(s, t.cbz, t.rbx, t.cbf);
-    t.staging_mb = (int)(staging_budget() >> 20);
+    t.staging_mb = (int)(staging_budget(true) >> 20);
     t.col_waves = 1;
     return t;
 }
@@ -579,9 +584,11 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
     // environment, else the tuned entry of a single-class plan, else defaults
     TuneParams tuned;
     const bool have_tuned = ncls == 1 && tune_lookup(rep[0]->Mz, rep[0]->Mx, rep[0]->nyu, tuned);
-    size_t l2_budget = staging_budget();
+    const bool lone = insts.size() == 1;
+    size_t l2_budget = staging_budget(lone);
     if (force && force->staging_mb > 0) l2_budget = (size_t)force->staging_mb << 20;
-    else if (!getenv("LH_STAGING_MB") && have_tuned && tuned.staging_mb > 0) l2_budget = (size_t)tuned.staging_mb << 20;
+    else if (!getenv("LH_STAGING_MB") && have_tuned && tuned.staging_mb > 0)  // tuned alone: a batch shares L2
+        l2_budget = lone ? (size_t)tuned.staging_mb << 20 : std::min(l2_budget, (size_t)tuned.staging_mb << 20);
     std::vector<int> chunk_eff(insts.size());
     for (size_t q = 0; q < insts.size(); q++) {
         const HostSetup &s = insts[q]->hs;
@@ -601,6 +608,11 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
         // launches (16^2 x 44 24.2 -> 22.6 us a substep, x 97 28.8 -> 27.4, 32^2 x
         // 97 34.2 -> 33.5, x 153 44.6 -> 46.1)
         if (fast && insts.size() == 1 && insts[q]->inst.chunk >= s.nyu && (long)s.nc * s.nyu <= kOneRoundRows) c = s.nyu;
+        // and a larger one as many rounds on each stream, of about the same size
+        if (fast && lone && c < (size_t)s.nyu) {
+            const size_t n = ((s.nyu + c - 1) / c + kRoundStreams - 1) / kRoundStreams * kRoundStreams;
+            c = (s.nyu + n - 1) / n;
+        }
         if (tiles[cls_of[q]].small) c = s.nyu;  // no staging: one round
         chunk_eff[q] = (int)c;
         rounds = std::max(rounds, (s.nyu + chunk_eff[q] - 1) / chunk_eff[q]);

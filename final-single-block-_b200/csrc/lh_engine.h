@@ -21,7 +21,7 @@ struct Tiles {
     int chunk = 32;    // planes per staging chunk
 };
 
-Tiles default_tiles(int Mx, int Mz, int nxh, int nyu);
+Tiles default_tiles(int Mx, int Mz, int nxh, int nyu, bool lone = false);
 size_t smem_zinv(const Tiles &t, int Mz);
 size_t smem_x(const Tiles &t, int Mx);
 size_t smem_zfwd(const Tiles &t, int Mz);

@@ -196,7 +196,7 @@ extern "C" int lh_autotune(lh_ctx *c, int force, int *params)
             axes.push_back({&TuneParams::rbx, {std::max(1, d0.rbx / 2), d0.rbx * 2}});
             axes.push_back({&TuneParams::cbf, {std::max(1, d0.cbf - 2), std::max(1, d0.cbf - 1), d0.cbf + 1}});
         }
-        axes.push_back({&TuneParams::staging_mb, {48, 64}});
+        axes.push_back({&TuneParams::staging_mb, {48, 64, 96}});
         if (!plan.column.empty()) axes.push_back({&TuneParams::col_waves, {2, 3, 4}});  // not on tiles
         for (auto &ax : axes) {
             for (int v : ax.second) {
