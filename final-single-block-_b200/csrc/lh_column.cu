@@ -53,60 +53,39 @@ __device__ __forceinline__ void cp8(double *s, const double *g)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_addr(s)), "l"(g));
 }
-// L2 eviction hints (LH_COLUMN_HINTS, compile time; 0 = none): 1 marks the
-// forward sweep's read-once rows (Nu_old, the Nu x/z parts, the y fluxes)
-// and the Nu and psi rows no later sweep of the launch reads as evict-first;
-// 2 also marks the rows the later sweeps read back (eliminated rows, factors,
-// the forward Poisson sweep) as evict-last.
-#ifndef LH_COLUMN_HINTS
-#define LH_COLUMN_HINTS 0
-#endif
+// L2 eviction hints: first marks the forward sweep's read-once rows (Nu_old, the Nu
+// x/z parts, the y fluxes) and the Nu and psi rows that no later sweep of the launch
+// reads, last the rows that the later sweeps read back (eliminated rows, factors, the
+// forward Poisson sweep).  The pass is bound by HBM (40 F of traffic asked for, F one
+// complex field, of which 32 reached it): column pass on B200, us, without -> with,
+// 128x128x153 133 -> 126, 192x192x257 482 -> 460, 256x256x257 867 -> 838, and the plane
+// pass keeps its times; the substep of 64 channels of 32x32x153 1258 -> 1238.  The
+// first kind alone 131, 479, 867.
 struct Hints {
     unsigned long long first, last;
     __device__ Hints()
     {
-        first = last = 0ull;
-#if LH_COLUMN_HINTS >= 1
         asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
-#endif
-#if LH_COLUMN_HINTS >= 2
         asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(last));
-#endif
     }
     __device__ __forceinline__ void cp_once(double2 *s, const double2 *g) const
     {
-#if LH_COLUMN_HINTS >= 1
         asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;\n" ::"r"(smem_addr(s)), "l"(g),
                      "l"(first));
-#else
-        cp16(s, g);
-#endif
     }
     __device__ __forceinline__ void st_once(double2 *g, double2 v) const
     {
-#if LH_COLUMN_HINTS >= 1
         asm volatile("st.global.L2::cache_hint.v2.f64 [%0], {%1, %2}, %3;" ::"l"(g), "d"(v.x), "d"(v.y), "l"(first)
                      : "memory");
-#else
-        *g = v;
-#endif
     }
     __device__ __forceinline__ void st_back(double2 *g, double2 v) const
     {
-#if LH_COLUMN_HINTS >= 2
         asm volatile("st.global.L2::cache_hint.v2.f64 [%0], {%1, %2}, %3;" ::"l"(g), "d"(v.x), "d"(v.y), "l"(last)
                      : "memory");
-#else
-        *g = v;
-#endif
     }
     __device__ __forceinline__ void st_back(double *g, double v) const
     {
-#if LH_COLUMN_HINTS >= 2
         asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(g), "d"(v), "l"(last) : "memory");
-#else
-        *g = v;
-#endif
     }
 };
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
