@@ -54,19 +54,17 @@ extern "C" int lh_ctx_create(const lh_grid_desc *desc, lh_ctx **out)
     }
     cudaError_t e = cudaGetDevice(&c->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMallocHost(&c->h_err, sizeof(int));
     if (e != cudaSuccess) {
-        if (c->st) cudaStreamDestroy(c->st);
         delete c;
         return LH_ECUDA;
     }
     const HostSetup &s = c->dev.hs;
     // the larger staging of a lone instance where the device has room to spare
-    Tiles t = default_tiles(s.Mx, s.Mz, s.nxh, s.nyu, true);
+    Tiles t = default_tiles(s.Mx, s.Mz, s.nxh, s.nyu), big = default_tiles(s.Mx, s.Mz, s.nxh, s.nyu, true);
     size_t room = 0, total = 0;
-    if (cudaMemGetInfo(&room, &total) != cudaSuccess || room / 2 < instance_bytes(s, t.chunk)) {
-        cudaGetLastError();
-        t = default_tiles(s.Mx, s.Mz, s.nxh, s.nyu);
+    if (big.chunk > t.chunk) {
+        if (cudaMemGetInfo(&room, &total) != cudaSuccess) cudaGetLastError();
+        else if (room / 2 >= instance_bytes(s, big.chunk)) t = big;
     }
     const char *gen = getenv("LH_GENERIC_FFT");
     e = instance_alloc(c->dev, t.chunk, c->st);
@@ -96,7 +94,6 @@ extern "C" int lh_ctx_destroy(lh_ctx *c)
     stats_release(c->stats_scr);
     instance_free(c->dev);
     if (c->st) cudaStreamDestroy(c->st);
-    if (c->h_err) cudaFreeHost(c->h_err);
     if (c->h_bounce) cudaFreeHost(c->h_bounce);
     for (cudaEvent_t ev : c->ev_bounce)
         if (ev) cudaEventDestroy(ev);
@@ -173,13 +170,14 @@ extern "C" int lh_download_nu(lh_ctx *c, double *nu1, double *nu2, double *nu3)
     return LH_OK;
 }
 
-// Waits for the stream and looks at the error word, which lands in page-locked
-// memory (a copy to pageable memory waits by itself).
+// Looks at the error word; the copy into pageable memory waits for the stream.  (A
+// page-locked word would take 3 us less here and 2 ms more at every creation.)
 static int check_err_word(lh_ctx *c)
 {
-    CK(cudaMemcpyAsync(c->h_err, c->dev.inst.err, sizeof(int), cudaMemcpyDeviceToHost, c->st), "error word");
+    int h = 0;
+    CK(cudaMemcpyAsync(&h, c->dev.inst.err, sizeof(int), cudaMemcpyDeviceToHost, c->st), "error word");
     CK(cudaStreamSynchronize(c->st), "synchronize");
-    if (*c->h_err & ERR_NONFINITE) return fail(c, LH_EDEVICE, "non-finite values in the state (time step unstable?)");
+    if (h & ERR_NONFINITE) return fail(c, LH_EDEVICE, "non-finite values in the state (time step unstable?)");
     return LH_OK;
 }
 

@@ -12,7 +12,6 @@ struct lh_ctx {
     lh::Plan plan;
     lh::Inst *d_inst = nullptr;
     cudaStream_t st = nullptr;
-    int *h_err = nullptr;      // page-locked copy of the error word
     char *h_bounce = nullptr;  // page-locked pieces of a large pageable download, on first use
     cudaEvent_t ev_bounce[2] = {nullptr, nullptr};
     int device = 0;            // the CUDA device current at lh_ctx_create

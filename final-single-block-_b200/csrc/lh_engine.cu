@@ -434,9 +434,9 @@ constexpr long kOneRoundRows = 60000;
 // (LH_SMALL_COLUMNS overrides): an SM takes 8 columns at a time, so 1184 are one
 // wave of about 5 + 4.5 rows/32 us, against 0.6 us a row of k_column, whatever
 // its columns: three waves from 64 rows on, two below.  Substep on B200, us,
-// k_column / tiles: 2112 columns x 44 rows 58.5 / 56.8, 2664 x 44 111 / 121;
-// 2664 x 97 222 / 216, x 153 343 / 324, x 257 593 / 552; 4704 x 97 174 / 190,
-// x 153 274 / 280, x 257 449 / 442; 28 channels of 144 x 97 185 / 204.
+// k_column / tiles: 2112 columns x 44 rows 53 / 53.5, 2664 x 44 60 / 71; 2664 x 97
+// 119 / 115, x 153 175 / 157, x 257 285 / 251; 4704 x 97 150 / 169, x 153 229 / 239,
+// x 257 384 / 381; 28 channels of 144 x 97 185 / 204.
 static long tile_columns(int max_nyu) { return (max_nyu < 64 ? 2 : 3) * 1184L; }
 
 // ---------------------------------------------------------------------------

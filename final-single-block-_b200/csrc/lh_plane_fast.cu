@@ -134,14 +134,16 @@ __global__ void __launch_bounds__(LH_ZINV_T, LH_MINB(NZ, LH_ZINV_B)) k_zinv_f(co
 // x transforms and products of one (plane j, block of rb z rows): xrow on rows
 // gathered from Sin with the y interpolations (interp_v FOU3D.f90:407, interp_u
 // :387): u1(j), u3(j); u2 at centre j, u2(j); u1, u3 at face j -> Sprod[slot]
-// What bounds it: the FP64 pipe, 48 % busy (55 % on the busiest SM), at the
-// warps that 168 registers leave (three CTAs of 128); then the L2 gather and the
-// launch's last wave.  x products alone, us a substep on B200, before (one
-// vector a half warp, or block-synchronous where vectors do not fit a warp) ->
-// now: 64^2 x 153 72 -> 61, 128^2 x 153 231 -> 183, 192^2 x 257 958 -> 900, 256^2
-// x 257 1955 -> 1340; the substep 128 -> 114, 401 -> 362, 1639 -> 1548, 3258 -> 2695.
-// Four CTAs an SM (128 registers) spill: 372 us at 128^2, 1764 at 192^2; three
-// instead of two at Mx = 384 3150.
+// What bounds it: the shared-memory / L1 data pipe (57 % of its cycles at Mx = 192)
+// and the FP64 pipe (50 %), at the warps that 168 registers leave (three CTAs of
+// 128).  x products alone, us a substep on B200 at 96 MB of staging: one vector a half
+// warp, or block-synchronous where vectors do not fit a warp -> products in registers
+// -> tasks packed on consecutive lanes: 64^2 x 153 72 -> 61 -> 57, 128^2 x 153 231 ->
+// 188 -> 181, 192^2 x 257 958 -> 910 -> 850, 256^2 x 257 1955 -> 1310 -> 1275; the substep
+// 128 -> 114 -> 110, 401 -> 363 -> 357, 1639 -> 1554 -> 1505, 3258 -> 2685 -> 2640.  Before
+// the packing, four CTAs an SM (128 registers) spilled: 372 us at 128^2, 1764 at
+// 192^2; three instead of two at Mx = 384 3150.  Two at N2 = 18: 192^2 x 257 706 for 641
+// (300 MB).
 template <int NX>
 __global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 6 ? 4 : (XPlan<NX>::N2 <= 18 ? 3 : 2))
     k_xprod_r(const Inst *__restrict__ insts, const Work *__restrict__ work, int rb, int want_max)
