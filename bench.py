@@ -226,7 +226,7 @@ def substep_alg_bytes(desc):
 
 # HBM bytes each kernel class of this design moves per substep, in units of
 # F: the z-inverse reads the three velocity planes, the x-products kernel
-# works on the L2-resident staging only, the z-forward writes the x/z parts
+# works on the staging only, the z-forward writes the x/z parts
 # of Nu and the three y-flux spectra, the column pass reads 13 fields and
 # writes 7 (u1 u2 u3 p, Nu x3).
 FIELD_PASSES = {"z_inverse": 3, "x_products": 0, "z_forward": 6, "dt": 0, "column": 20}

@@ -134,8 +134,8 @@ __global__ void __launch_bounds__(LH_ZINV_T, LH_MINB(NZ, LH_ZINV_B)) k_zinv_f(co
 // x transforms and products of one (plane j, block of rb z rows): xrow on rows
 // gathered from Sin with the y interpolations (interp_v FOU3D.f90:407, interp_u
 // :387): u1(j), u3(j); u2 at centre j, u2(j); u1, u3 at face j -> Sprod[slot]
-// What bounds it: the shared-memory / L1 data pipe (57 % of its cycles at Mx = 192)
-// and the FP64 pipe (50 %), at the warps that 168 registers leave (three CTAs of
+// What bounds it: the FP64 pipe (51 % of its cycles at Mx = 192) and the shared-memory
+// / L1 data pipe (50 %), at the warps that 168 registers leave (three CTAs of
 // 128).  x products alone, us a substep on B200 at 96 MB of staging: one vector a half
 // warp, or block-synchronous where vectors do not fit a warp -> products in registers
 // -> tasks packed on consecutive lanes: 64^2 x 153 72 -> 61 -> 57, 128^2 x 153 231 ->
@@ -220,7 +220,10 @@ __global__ void __launch_bounds__(kXprodThreads, XPlan<NX>::N2 <= 6 ? 4 : (XPlan
 // phys_to_four_du's cft (FOU3D.f90:1654-1672), der_x/der_z (:420-523) and
 // planes_to_modes_UVP/NUVP.  The six products split into two independent
 // halves: {uu, uw, ww} -> Nu1 and Nu3 x/z parts; {vv, uv, wv} -> vv_c, uv_f,
-// wv_f and the Nu2 x/z part.
+// wv_f and the Nu2 x/z part.  What bounds it: the loads' latency at 22 warps an SM
+// and the shared-memory / L1 data pipe (51 % of its cycles at Mz = 192; 56 % while the
+// second pass read across banks), whose segments of cb modes are 64 bytes there; wider
+// CTAs (up to 512 threads, cb = 10) leave the substep within 2 % or slower.
 template <int NZ>
 __global__ void __launch_bounds__(LH_ZFWD_T, LH_MINB(NZ, LH_ZFWD_B)) k_zfwd_f(const Inst *__restrict__ insts, const Work *__restrict__ work,
                                                          int count, int cb)

@@ -55,11 +55,12 @@ struct TwStep {
 //
 // A vector crosses shared memory twice (the exchanges, 4 accesses an element)
 // instead of 12 accesses when the gather, the products and the split went
-// through it too.  That pipe is still the busiest (57 % of its cycles at Mx = 192,
+// through it too.  That pipe was still the busiest (57 % of its cycles at Mx = 192,
 // against the FP64 pipe's 50 %), so the tasks of as many whole rows as fit sit on
-// consecutive lanes (24 of 32 at N2 = 12; spread over the rows' own lanes they
-// touched a quarter of a wavefront more), m -> N2 - m stays inside the row, and the
-// matrices of neighbouring rows are a task's columns apart in the banks.  A lane
+// consecutive lanes (24 of 32 at N2 = 12; on the rows' own lanes they took four
+// wavefronts an access instead of three), m -> N2 - m stays inside the row, and the
+// matrices of neighbouring rows are a task's columns apart in the banks (now 50 % and
+// 51 %, wavefronts of a substep at 128^2 x 153 21.5 -> 18.3 million).  A lane
 // keeps its columns of the matrix from one use to the next, so two __syncwarp a
 // vector are all the synchronisation.  Every load of a task is issued before the
 // first is used: loaded mode by mode the stage waited on L2 for half its time.
