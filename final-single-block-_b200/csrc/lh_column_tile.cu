@@ -19,8 +19,8 @@
 // code the pass was half again as slow).  Column pass alone, us a substep on
 // B200, k_column -> tiles: 32x32x153 86 -> 23, 64x64x153 94 -> 51, 96x64x129
 // 85 -> 65; the whole substep, with the per-column kernel that served up to 1536
-// columns before the tiles in brackets: 16x16x97 66 [30] -> 28, 32x32x153 105
-// [52] -> 44, 32x32x257 166 [104] -> 66, 64x64x153 168 -> 127.  Larger plans keep
+// columns before the tiles in brackets: 16x16x97 61 [30] -> 24, 32x32x153 99
+// [52] -> 41, 32x32x257 156 [104] -> 59, 64x64x153 149 -> 111.  Larger plans keep
 // k_column, whose streaming sweeps move half again as many rows once they fill
 // the GPU (tile_columns, lh_engine.cu).
 //

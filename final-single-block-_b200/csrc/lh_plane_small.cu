@@ -19,10 +19,11 @@
 //
 // What bounds it: latency at two CTAs an SM (the plane's 78 KB and the row
 // matrices), then the FP64 pipe, 35 % busy.  B200, us a substep, staged -> here:
-// 64 channels of 32 x 32 x 153 1539 -> 1260, 16 of them 370 -> 330, 16 x 16 x 153
-// alone 33.7 -> 30.9; 32 x 32 x 153 alone, whose 152 planes leave four SMs with
-// two, 40.9 -> 46.8 (small_plane_pays decides).  288, 320 and 384 threads: 1405,
-// 1435, 1561 us for the 64 (96 and 80 registers spill).
+// 64 channels of 32 x 32 x 153 1515 -> 1239, 16 of them 370 -> 323, 3 of them 92 -> 86, 2
+// 58 -> 63; 16 x 16 x 153 alone 33.7 -> 31.5, x 97 28.0 -> 24.5; 32 x 32 x 153 alone,
+// whose 152 planes leave four SMs with two, 41.3 -> 46.9 (small_plane_pays decides).
+// 288, 320 and 384 threads: 1405, 1435, 1561 us for the 64 where 256 took 1260 (96 and
+// 80 registers spill).
 #include "lh_fft.cuh"
 #include "lh_kernels.cuh"
 #include "lh_xprod.cuh"
