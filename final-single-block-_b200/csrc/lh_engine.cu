@@ -807,7 +807,12 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
     if (gz && (e = raise_smem_limit((const void *)k_zinv, gz)) != cudaSuccess) return e;
     if (gx && (e = raise_smem_limit((const void *)k_xprod, gx)) != cudaSuccess) return e;
     if (gf && (e = raise_smem_limit((const void *)k_zfwd, gf)) != cudaSuccess) return e;
-    p.sm_factors = 3 * (size_t)(max_nyu + 1) * sizeof(double);
+    // k_factors holds the metrics of the tiled instances only, whose rows fit a tile (970
+    // at most), so it stays below the 48 KB a launch may ask for without a raised limit
+    int tiled_nyu = 0;
+    for (size_t q = 0; q < insts.size(); q++)
+        if (width[q] != 0) tiled_nyu = std::max(tiled_nyu, insts[q]->hs.nyu);
+    p.sm_factors = 3 * (size_t)(tiled_nyu + 1) * sizeof(double);
     for (const Plan::ColLaunch &t : p.col_tiles)
         if ((e = column_tile_attributes(t.C, t.smem)) != cudaSuccess) return e;
     if (!sequential) return cudaSuccess;

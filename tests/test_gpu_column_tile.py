@@ -66,3 +66,27 @@ def test_noalloc_solve_at_the_row_limits(Nx, Nz, ny, grid):
     assert e.L.lh_lusolu_noalloc(e.h, grid, 2, d.dt, x.data_ptr(), x.data_ptr()) == 0
     e.synchronize()
     assert rel_l2(x.cpu().numpy().T, want) <= 1e-13
+
+
+def test_tiles_beside_an_instance_they_do_not_serve():
+    """One plan with tiled columns and with columns too tall for a tile: the rows of
+    the tall instance do not size the tiles' factors, and each instance steps as it
+    does alone (8 columns a tile in both plans; k_column in both)."""
+    import numpy as np
+    from lh_b200 import Batch, Desc, Engine, grids, perturbed_laminar
+    descs = [Desc(Nx=64, Nz=64, ny=97, dt_mode=1, dt=1e-4), Desc(Nx=8, Nz=8, ny=1700, dt_mode=1, dt=1e-5)]
+    ics = [perturbed_laminar(d, 60 + k, *grids(d)) for k, d in enumerate(descs)]
+    b = Batch()
+    slots = [b.add(d, *ic) for d, ic in zip(descs, ics)]
+    b.step(2)
+    b.synchronize()
+    for d, s, ic in zip(descs, slots, ics):
+        e = Engine(d)
+        e.upload(*ic)
+        e.step(2)
+        e.synchronize()
+        want, got = e.download(), b.download(s)
+        for f in ("u1", "u2", "u3", "p"):
+            assert np.isfinite(want[f]).all() and np.array_equal(got[f], want[f]), f
+        e.close()
+    b.close()
