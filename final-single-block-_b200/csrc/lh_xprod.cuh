@@ -189,11 +189,13 @@ __device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int rows, bo
             }
         }
         __syncwarp();
-        // inverse pass 2, products, forward pass 1 of this lane's row of the matrix
+        // inverse pass 2, products, forward pass 1 of this lane's row of the matrix.  Lanes
+        // left over (N1 = 6, 12) take no part: rows are overwritten here without a barrier,
+        // so nobody but their lanes may read them, and zeros leave the maxima alone.
         {
             double2 b[N2];
 #pragma unroll
-            for (int n2 = 0; n2 < N2; n2++) b[n2] = Tr[n2];
+            for (int n2 = 0; n2 < N2; n2++) b[n2] = on ? Tr[n2] : make_double2(0.0, 0.0);
             DFT<N2, +1, NX>::run(b, tw);
             if (pair == 0) {
 #pragma unroll
@@ -231,11 +233,13 @@ __device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int rows, bo
         for (int g = 0; g < ROUNDS; g++) {
             const Task q(g, lane_row, lane_task, r, on, rows);
             const int m = q.m;
-            // packed lanes without a task read nothing, others their row's first column
+            // lanes without a task read nothing, those of a row without one their row's
+            // first column
+            const bool reads = PACKED ? q.on : on;
             const double2 *const Tm = T + (q.row * RS + (m >= 0 ? m : 0));
             double2 e[N1];
 #pragma unroll
-            for (int k1 = 0; k1 < N1; k1++) e[k1] = !PACKED || q.on ? Tm[k1 * LD] : make_double2(0.0, 0.0);
+            for (int k1 = 0; k1 < N1; k1++) e[k1] = reads ? Tm[k1 * LD] : make_double2(0.0, 0.0);
             DFT<N1, -1, NX>::run(e, tw);
             const double h = 0.5 / NX;
 #pragma unroll
