@@ -42,12 +42,16 @@ size_t staging_units(int chunk) { return (size_t)(chunk + 2 * kRoundStreams) * 3
 // worth more.  Substep on B200, us, 96 / 150 / 200 / 300 / 500 MB: 128x128x153 357 354
 // 355 351 352, 192x192x257 1502 1478 1467 1452 1442, 256x256x257 2642 2629 2616 2613
 // 2604, 216x216x129 1026 975 971 971 969; an odd number of rounds loses up to 5 %.
+// Not where the generic plane kernels run, which are slower so: 288x288x65 2408 us at
+// 96 MB, 2496 at 300, 384x384x33 2133 and 2213, 288x96x65 742 and 747.
 size_t staging_budget(bool lone)
 {
     const char *ev = getenv("LH_STAGING_MB");
     const long mb = ev ? atol(ev) : 0;
     return (size_t)(mb > 0 ? mb : lone ? 300 : 96) << 20;
 }
+
+bool compiled_planes(const HostSetup &hs) { return fast_size(hs.Mz) && fast_size(hs.Mx); }
 
 Tiles default_tiles(int Mx, int Mz, int nxh, int nyu, bool lone)
 {
@@ -500,7 +504,7 @@ void default_bounds(const HostSetup &s, int &cbz, int &rbx, int &cbf)
 ClassTiles class_tiles(const HostSetup &s, bool force_generic, const TuneParams *force)
 {
     ClassTiles c{};
-    c.fast = !force_generic && fast_size(s.Mz) && fast_size(s.Mx);
+    c.fast = !force_generic && compiled_planes(s);
     if (c.fast) {
         int a = 0, b = 0, d = 0;
         default_bounds(s, a, b, d);
@@ -538,8 +542,8 @@ ClassTiles class_tiles(const HostSetup &s, bool force_generic, const TuneParams 
 TuneParams default_params(const HostSetup &s)
 {
     TuneParams t;
-    if (fast_size(s.Mz) && fast_size(s.Mx)) default_bounds(s, t.cbz, t.rbx, t.cbf);
-    t.staging_mb = (int)(staging_budget(true) >> 20);
+    if (compiled_planes(s)) default_bounds(s, t.cbz, t.rbx, t.cbf);
+    t.staging_mb = (int)(staging_budget(compiled_planes(s)) >> 20);
     t.col_waves = 1;
     return t;
 }
@@ -585,7 +589,7 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
     TuneParams tuned;
     const bool have_tuned = ncls == 1 && tune_lookup(rep[0]->Mz, rep[0]->Mx, rep[0]->nyu, tuned);
     const bool lone = insts.size() == 1;
-    size_t l2_budget = staging_budget(lone);
+    size_t l2_budget = staging_budget(lone && tiles[0].fast);
     if (force && force->staging_mb > 0) l2_budget = (size_t)force->staging_mb << 20;
     else if (!getenv("LH_STAGING_MB") && have_tuned && tuned.staging_mb > 0)  // tuned alone: a batch shares L2
         l2_budget = lone ? (size_t)tuned.staging_mb << 20 : std::min(l2_budget, (size_t)tuned.staging_mb << 20);

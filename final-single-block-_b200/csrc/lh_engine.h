@@ -21,6 +21,8 @@ struct Tiles {
     int chunk = 32;    // planes per staging chunk
 };
 
+// whether the plane kernels of an instance are the compiled ones (lh_plane_fast.cu)
+bool compiled_planes(const HostSetup &hs);
 Tiles default_tiles(int Mx, int Mz, int nxh, int nyu, bool lone = false);
 size_t smem_zinv(const Tiles &t, int Mz);
 size_t smem_x(const Tiles &t, int Mx);
