@@ -164,7 +164,7 @@ extern "C" size_t lh_instance_bytes(const lh_grid_desc *desc)
     HostSetup hs;
     if (!build_setup(*desc, hs).empty()) return 0;
     Tiles t = default_tiles(hs.Mx, hs.Mz, hs.nxh, hs.nyu);
-    return instance_bytes(hs, t.chunk);
+    return instance_bytes(hs, t.chunk, true);
 }
 
 extern "C" int lh_batch_add(lh_batch *b, const lh_grid_desc *desc, const double *u1, const double *u2,
@@ -177,7 +177,7 @@ extern "C" int lh_batch_add(lh_batch *b, const lh_grid_desc *desc, const double 
     std::string why = build_setup(*desc, d->hs);
     if (!why.empty()) return bfail(b, LH_EINVAL, why);
     Tiles t = default_tiles(d->hs.Mx, d->hs.Mz, d->hs.nxh, d->hs.nyu);
-    const size_t need = instance_bytes(d->hs, t.chunk);
+    const size_t need = instance_bytes(d->hs, t.chunk, true);
     if (b->budget && b->used + need > b->budget)
         return bfail(b, LH_ENOMEM, "HBM budget exhausted");
     // The new instance is allocated and uploaded on the admission stream
@@ -199,11 +199,11 @@ extern "C" int lh_batch_add(lh_batch *b, const lh_grid_desc *desc, const double 
     } else if (b->budget) {
         pool_release(b, b->budget > b->used + need ? b->budget - b->used - need : 0);
     }
-    cudaError_t e = instance_alloc(*d, t.chunk, b->st_up, reuse, reuse_bytes);
+    cudaError_t e = instance_alloc(*d, t.chunk, true, b->st_up, reuse, reuse_bytes);
     if (e == cudaErrorMemoryAllocation && !reuse && !b->pool.empty()) {
         cudaGetLastError();
         pool_release(b, 0);
-        e = instance_alloc(*d, t.chunk, b->st_up);
+        e = instance_alloc(*d, t.chunk, true, b->st_up);
     }
     if (e == cudaSuccess) e = instance_upload(*d, u1, u2, u3, p, b->st_up);
     if (e != cudaSuccess) {

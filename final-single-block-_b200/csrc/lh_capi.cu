@@ -61,15 +61,8 @@ extern "C" int lh_ctx_create(const lh_grid_desc *desc, lh_ctx **out)
     const HostSetup &s = c->dev.hs;
     const char *gen = getenv("LH_GENERIC_FFT");
     const bool generic = gen && gen[0] == '1';
-    // the larger staging of a lone instance where the device has room to spare
-    Tiles t = default_tiles(s.Mx, s.Mz, s.nxh, s.nyu);
-    const Tiles big = default_tiles(s.Mx, s.Mz, s.nxh, s.nyu, !generic && compiled_planes(s));
-    size_t room = 0, total = 0;
-    if (big.chunk > t.chunk) {
-        if (cudaMemGetInfo(&room, &total) != cudaSuccess) cudaGetLastError();
-        else if (room / 2 >= instance_bytes(s, big.chunk)) t = big;
-    }
-    e = instance_alloc(c->dev, t.chunk, c->st);
+    const bool split = column_split_wanted();
+    e = instance_alloc(c->dev, lone_chunk(s, !generic && compiled_planes(s), split), split, c->st);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_inst, sizeof(Inst));
     if (e == cudaSuccess) e = cudaMemcpy(c->d_inst, &c->dev.inst, sizeof(Inst), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = plan_build(c->plan, {&c->dev}, generic);

@@ -37,11 +37,12 @@ size_t staging_units(int chunk) { return (size_t)(chunk + 2 * kRoundStreams) * 3
 
 // Bytes of plane staging one chunk round may use across all instances of a
 // plan, kept well inside the 126 MB L2 (LH_STAGING_MB overrides, for tuning).
-// A lone instance takes 300 MB: its rounds' staging then spills to HBM, which the
+// A lone instance takes up to 300 MB: its rounds' staging then spills to HBM, which the
 // plane pass leaves mostly idle, but fewer launches, each of several full waves, are
 // worth more.  Substep on B200, us, 96 / 150 / 200 / 300 / 500 MB: 128x128x153 357 354
 // 355 351 352, 192x192x257 1502 1478 1467 1452 1442, 256x256x257 2642 2629 2616 2613
-// 2604, 216x216x129 1026 975 971 971 969; an odd number of rounds loses up to 5 %.
+// 2604, 216x216x129 1026 975 971 971 969; an odd number of rounds loses up to 5 %.  It
+// never takes more memory than lh_instance_bytes states (lone_chunk).
 // Not where the generic plane kernels run, which are slower so: 288x288x65 2408 us at
 // 96 MB, 2496 at 300, 384x384x33 2133 and 2213, 288x96x65 742 and 747.
 size_t staging_budget(bool lone)
@@ -88,8 +89,9 @@ struct Carver {
     }
 };
 
-// Lay out every buffer of an instance; with base == nullptr it only sizes.
-void carve(const HostSetup &s, int chunk, Carver &c, Inst &I, double2 **stage, size_t *stage_elems)
+// Lay out every buffer of an instance; with base == nullptr it only sizes.  split: with
+// the rows that a split column pass needs.
+void carve(const HostSetup &s, int chunk, bool split, Carver &c, Inst &I, double2 **stage, size_t *stage_elems)
 {
     const size_t nc = s.nc, nu = s.nyu + 2, nv = s.nyv + 2, np = s.nyu;
     I.yu = c.take<double>(nu);
@@ -123,10 +125,12 @@ void carve(const HostSetup &s, int chunk, Carver &c, Inst &I, double2 **stage, s
     I.FACU = c.take<double>(nu * nc);
     I.FACV = c.take<double>(nv * nc);
     I.PSI = c.take<double2>(np * nc);
-    I.Y1 = c.take<double2>(nu * nc);
-    I.Y2 = c.take<double2>(nv * nc);
-    I.Y3 = c.take<double2>(nu * nc);
-    I.CARRY = c.take<double2>(18 * nc);
+    if (split) {
+        I.Y1 = c.take<double2>(nu * nc);
+        I.Y2 = c.take<double2>(nv * nc);
+        I.Y3 = c.take<double2>(nu * nc);
+        I.CARRY = c.take<double2>(18 * nc);
+    }
     I.U11 = c.take<double>(nu);
     I.F11 = c.take<double>(nu);
     I.S = c.take<double2>(staging_units(chunk) * s.Mz * s.nxh);
@@ -137,23 +141,36 @@ void carve(const HostSetup &s, int chunk, Carver &c, Inst &I, double2 **stage, s
 }
 }  // namespace
 
-size_t instance_bytes(const HostSetup &hs, int chunk)
+size_t instance_bytes(const HostSetup &hs, int chunk, bool split)
 {
     Carver c;
     Inst I{};
     double2 *st;
     size_t se;
-    carve(hs, chunk, c, I, &st, &se);
+    carve(hs, chunk, split, c, I, &st, &se);
     return c.off;
 }
 
-cudaError_t instance_alloc(DevInstance &d, int chunk, cudaStream_t st, void *reuse, size_t reuse_bytes)
+// A lone instance's larger staging stands where the rows of a split column pass would
+// be, which only LH_COLUMN_SPLIT=1 uses: what a caller planned by lh_instance_bytes
+// still fits.
+int lone_chunk(const HostSetup &hs, bool compiled, bool split)
+{
+    const int base = default_tiles(hs.Mx, hs.Mz, hs.nxh, hs.nyu).chunk;
+    if (!compiled || split) return base;
+    const size_t limit = instance_bytes(hs, base, true);
+    int chunk = std::max(base, default_tiles(hs.Mx, hs.Mz, hs.nxh, hs.nyu, true).chunk);
+    while (chunk > base && instance_bytes(hs, chunk, false) > limit) chunk--;
+    return chunk;
+}
+
+cudaError_t instance_alloc(DevInstance &d, int chunk, bool split, cudaStream_t st, void *reuse, size_t reuse_bytes)
 {
     const HostSetup &s = d.hs;
     Carver c;
     Inst &I = d.inst;
     memset(&I, 0, sizeof(I));
-    carve(s, chunk, c, I, &d.stage, &d.stage_elems);
+    carve(s, chunk, split, c, I, &d.stage, &d.stage_elems);
     d.bytes = c.off;
     cudaError_t e = cudaSuccess;
     if (reuse && reuse_bytes >= d.bytes) {
@@ -169,7 +186,7 @@ cudaError_t instance_alloc(DevInstance &d, int chunk, cudaStream_t st, void *reu
     }
     c = Carver();
     c.base = (char *)d.block;
-    carve(s, chunk, c, I, &d.stage, &d.stage_elems);
+    carve(s, chunk, split, c, I, &d.stage, &d.stage_elems);
     e = cudaMemsetAsync(d.block, 0, d.bytes, st);
     if (e != cudaSuccess) return e;
     auto up = [&](const void *dst, const void *src, size_t bytes) {
@@ -429,6 +446,11 @@ cudaError_t instance_download(DevInstance &d, double *u1, double *u2, double *u3
 // Whether the sequential column pass is split into forward-sweep chunks
 // beside the plane rounds (LH_COLUMN_SPLIT=0/1 overrides).
 constexpr bool kColumnSplitDefault = false;
+bool column_split_wanted()
+{
+    const char *cs = getenv("LH_COLUMN_SPLIT");
+    return cs ? cs[0] == '1' : kColumnSplitDefault;
+}
 
 // Lone instances of at most this many columns x rows run the plane pass in one
 // round (plan_build).
@@ -735,8 +757,8 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
     p.n_factors = all.size() - p.off_factors;
     // split column pass: per round, every instance's rows of that round x its
     // column blocks; plus one chunk of all rows
-    const char *cs = getenv("LH_COLUMN_SPLIT");
-    p.col_split = p.col_tiles.empty() && (cs ? cs[0] == '1' : kColumnSplitDefault);
+    p.col_split = p.col_tiles.empty() && column_split_wanted();
+    for (const DevInstance *d : insts) p.col_split &= d->inst.Y1 != nullptr;  // a lone context made without it
     p.col_a.assign(rounds, {0, 0});
     p.off_col_full = p.n_col_full = 0;
     if (p.col_split) {

@@ -21,6 +21,7 @@ struct Tiles {
     int chunk = 32;    // planes per staging chunk
 };
 
+bool column_split_wanted();
 // whether the plane kernels of an instance are the compiled ones (lh_plane_fast.cu)
 bool compiled_planes(const HostSetup &hs);
 Tiles default_tiles(int Mx, int Mz, int nxh, int nyu, bool lone = false);
@@ -43,11 +44,13 @@ struct DevInstance {
 // Plane fields of staging an instance allocates for `chunk` planes.
 size_t staging_units(int chunk);
 // Bytes one instance needs for a staging chunk of `chunk` planes.
-size_t instance_bytes(const HostSetup &hs, int chunk);
+size_t instance_bytes(const HostSetup &hs, int chunk, bool split);
+// planes of staging of a lone instance
+int lone_chunk(const HostSetup &hs, bool compiled, bool split);
 // Allocate and fill the device arrays of an instance (synchronous).
 // With `reuse` (a device block of reuse_bytes from an earlier instance) the
 // instance is carved from it when it is large enough, instead of cudaMalloc.
-cudaError_t instance_alloc(DevInstance &d, int chunk, cudaStream_t st, void *reuse = nullptr, size_t reuse_bytes = 0);
+cudaError_t instance_alloc(DevInstance &d, int chunk, bool split, cudaStream_t st, void *reuse = nullptr, size_t reuse_bytes = 0);
 void instance_free(DevInstance &d);
 // Upload / download the four state fields in the reference column layout.
 cudaError_t instance_upload(DevInstance &d, const double *u1, const double *u2, const double *u3, const double *p,

@@ -164,7 +164,7 @@ extern "C" int lh_autotune(lh_ctx *c, int force, int *params)
         Plan plan;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         const bool cfl = c->dev.desc.dt_mode == LH_DT_CFL;
-        cudaError_t e = instance_alloc(scr, c->dev.inst.chunk, c->st);
+        cudaError_t e = instance_alloc(scr, c->dev.inst.chunk, c->dev.inst.Y1 != nullptr, c->st);
         if (e == cudaSuccess && c->have_state) {
             // the current state, so the CFL time step is the run's
             const size_t nc = s.nc;
