@@ -68,6 +68,7 @@ extern "C" int lh_ctx_create(const lh_grid_desc *desc, lh_ctx **out)
     if (e == cudaSuccess) e = plan_build(c->plan, {&c->dev}, generic);
     if (e != cudaSuccess) {
         int code = e == cudaErrorMemoryAllocation ? LH_ENOMEM : LH_ECUDA;
+        cudaGetLastError();  // reported by the code: not left for the thread's next call
         lh_ctx_destroy(c);
         return code;
     }
@@ -318,14 +319,23 @@ static cudaError_t copy_out(lh_ctx *c, void *dst, const void *src, size_t bytes)
 {
     constexpr size_t kPiece = (size_t)1 << 20;
     cudaPointerAttributes at;
-    bool bounce = bytes >= kPiece / 4 && cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
-                  at.type == cudaMemoryTypeUnregistered;
-    if (bounce && !c->h_bounce) {
-        if (cudaMallocHost(&c->h_bounce, 2 * kPiece) != cudaSuccess) c->h_bounce = nullptr;
-        for (cudaEvent_t &ev : c->ev_bounce)
-            if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) ev = nullptr;
+    bool bounce = bytes >= kPiece / 4;
+    if (bounce && cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+        cudaGetLastError();
+        bounce = false;
     }
-    cudaGetLastError();
+    bounce = bounce && at.type == cudaMemoryTypeUnregistered;
+    if (bounce && !c->h_bounce) {
+        if (cudaMallocHost(&c->h_bounce, 2 * kPiece) != cudaSuccess) {
+            cudaGetLastError();
+            c->h_bounce = nullptr;
+        }
+        for (cudaEvent_t &ev : c->ev_bounce)
+            if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+                cudaGetLastError();
+                ev = nullptr;
+            }
+    }
     cudaError_t e = cudaSuccess;
     if (!bounce || !c->h_bounce || !c->ev_bounce[0] || !c->ev_bounce[1]) {
         e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->st);
@@ -371,9 +381,7 @@ extern "C" int lh_get_spectra(lh_ctx *c, int which, double *out, size_t cap, int
     // the device (a field of the staging holds two of the real arrays): strided
     // on the host it took five times the copy
     double *t = reinterpret_cast<double *>(c->dev.stage);
-    const dim3 grid((unsigned)((nc + 31) / 32), (unsigned)((rows + 31) / 32)), block(32, 8);
-    k_rows_to_cols<<<grid, block, 0, c->st>>>(c->d_spec + off * nc, t, (int)rows, (int)nc);
-    CK(cudaGetLastError(), "spectra layout");
+    CK(rows_to_cols(c->d_spec + off * nc, t, (int)rows, (int)nc, c->st), "spectra layout");
     CK(copy_out(c, out, t, n * sizeof(double)), "spectra download");
     return (int)n;
 }

@@ -773,6 +773,14 @@ __global__ void k_rows_to_cols(const double *__restrict__ src, double *__restric
     }
 }
 
+// The launch's own status: an error that an earlier call left on this thread is not this
+// transform's.
+cudaError_t rows_to_cols(const double *src, double *dst, int len, int nc, cudaStream_t st)
+{
+    void *args[] = {&src, &dst, &len, &nc};
+    return cudaLaunchKernel((const void *)k_rows_to_cols, dim3((nc + 31) / 32, (len + 31) / 32), dim3(32, 8), args, 0, st);
+}
+
 // ---------------------------------------------------------------------------
 // Stand-alone LUsolU on plane-major columns (unit entry): grid 2 = u/w
 // (rows 0..nyu+1), 1 = v (rows 0..nyv+1)

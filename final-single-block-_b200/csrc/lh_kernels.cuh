@@ -48,7 +48,7 @@ struct StateReset {
     double value[SC_COUNT];
 };
 cudaError_t reset_state(const StateReset &r, cudaStream_t st);
-__global__ void k_rows_to_cols(const double *__restrict__ src, double *__restrict__ dst, int len, int nc);
+cudaError_t rows_to_cols(const double *src, double *dst, int len, int nc, cudaStream_t st);
 __global__ void k_lusolu(const Inst *__restrict__ insts, int grid, int kRK, double dt, const double2 *rhs,
                          double2 *u, double *fac);
 // the same without global scratch where the rows fit the lanes (lh_column_tile.cu)

@@ -117,3 +117,26 @@ def test_pageable_downloads(N):
         assert e.L.lh_download_state(e.h, *[_dp(x) for x in b]) == 0
     assert all(np.array_equal(x, y) for x, y in zip(*got))
     e.close()
+
+
+def test_spectra_after_a_refused_context():
+    """A context that cannot be made (columns of 2600 rows do not fit the column pass):
+    its error is not the next fetch's of another context, nor its next upload's."""
+    from lh_b200 import Desc, Engine
+    from lh_b200.capi import LHError
+    e = Engine(Desc(Nx=16, Nz=16, ny=33, dt_mode=1, dt=1e-4))
+    s = e.sizes
+    rng = np.random.default_rng(6)
+    e.upload(*[1e-3 * (rng.standard_normal((s.ncols, n)) + 1j * rng.standard_normal((s.ncols, n)))
+               for n in (s.nyu + 2, s.nyv + 2, s.nyu + 2, s.nyu)])
+    e.spectra_accumulate()
+    want, _ = e.spectra()
+    with pytest.raises(LHError):
+        Engine(Desc(Nx=8, Nz=8, ny=2600, dt_mode=1, dt=1e-4))
+    got, _ = e.spectra()
+    for k in want:
+        assert want[k].any() and np.array_equal(got[k], want[k]), k
+    with pytest.raises(LHError):
+        Engine(Desc(Nx=8, Nz=8, ny=2600, dt_mode=1, dt=1e-4))
+    e.upload(*[np.zeros((s.ncols, n), dtype=complex) for n in (s.nyu + 2, s.nyv + 2, s.nyu + 2, s.nyu)])
+    e.close()
