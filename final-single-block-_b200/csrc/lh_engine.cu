@@ -987,7 +987,7 @@ cudaError_t launch_substep(const Plan &p, const Inst *d_insts, int kRK, bool cfl
     if (p.n_factors && !f_beside) {
         time_begin(timer, st);
         factors_launch((unsigned)p.n_factors, p.sm_factors, st, d_insts, p.d_work + p.off_factors, kRK);
-        if ((e = time_end(timer, 3, st)) != cudaSuccess) return e;
+        if ((e = time_end(timer, 4, st)) != cudaSuccess) return e;
     }
     time_begin(timer, st);
     if (p.col_split) {

@@ -90,3 +90,16 @@ def test_tiles_beside_an_instance_they_do_not_serve():
             assert np.isfinite(want[f]).all() and np.array_equal(got[f], want[f]), f
         e.close()
     b.close()
+
+
+def test_profile_counts_the_factors_as_column_pass():
+    """dt is one launch a step; the tiles' factors belong to the column pass, two launches
+    a substep with it."""
+    from lh_b200 import Desc, Engine, grids, perturbed_laminar
+    for cfl in (False, True):
+        d = Desc(Nx=16, Nz=16, ny=33, dt_mode=0 if cfl else 1, dt=1e-3, CFL=0.5)
+        e = Engine(d)
+        e.upload(*perturbed_laminar(d, 71, *grids(d)))
+        prof = e.profile(2)
+        assert prof["dt"][1] == 2 and prof["column"][1] == 12, prof
+        e.close()
