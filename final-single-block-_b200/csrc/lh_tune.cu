@@ -13,8 +13,8 @@
 //
 // Results live in a process-wide table (plan_build consults it for every
 // size class, single instances and batches alike) and in a text cache file,
-// one line per entry keyed by the GPU's name and the sizes:
-//   <gpu name>|<Mz>|<Mx>|<nyu> <cbz> <rbx> <cbf> <staging_mb> <col_waves> <ms per step>
+// one line per entry keyed by the GPU's name, the version of the kernels and the sizes:
+//   <gpu name>|k<version>|<Mz>|<Mx>|<nyu> <cbz> <rbx> <cbf> <staging_mb> <col_waves> <ms per step>
 // The file is LH_TUNE_CACHE, else lh_tune_cache.txt beside the library.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
@@ -84,10 +84,15 @@ std::string gpu_name()
     return n;
 }
 
+// Raised whenever the kernels' shapes or their defaults change: what was measured with
+// others is measured again.  1 (no version in the key): staging of at most 96 MB and an
+// x stage of other rows per CTA, which capped today's defaults.
+constexpr int kKernelVersion = 2;
+
 std::string cache_key(const HostSetup &s)
 {
     char b[128];
-    snprintf(b, sizeof b, "|%d|%d|%d", s.Mz, s.Mx, s.nyu);
+    snprintf(b, sizeof b, "|k%d|%d|%d|%d", kKernelVersion, s.Mz, s.Mx, s.nyu);
     return gpu_name() + b;
 }
 

@@ -119,8 +119,9 @@ int lh_get_stream(lh_ctx *ctx, void **stream);
  * context's size, chosen by timing RK3 steps of a scratch instance (the
  * context's state is not touched; its current state is copied in so the CFL
  * step is the run's).  None of them changes any arithmetic: the states stay
- * bit-identical.  Results are cached per GPU name and (Mz, Mx, nyu) in the
- * file LH_TUNE_CACHE (default lh_tune_cache.txt beside the library) and in a
+ * bit-identical.  Results are cached per GPU name, version of the kernels and
+ * (Mz, Mx, nyu) in the file LH_TUNE_CACHE (default lh_tune_cache.txt beside
+ * the library; entries of other versions are measured again) and in a
  * process-wide table that every later plan of that size -- contexts and
  * batches -- uses.  force = 1 measures even when the cache has the size.
  * params (may be NULL) receives [cbz, rbx, cbf, staging_mb, col_waves,

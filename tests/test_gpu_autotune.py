@@ -50,3 +50,19 @@ def test_autotune_measures_caches_and_keeps_states(tmp_path, monkeypatch):
     for f in FIELDS:
         assert np.array_equal(got_b[f], want[f]), f
     b.close()
+
+
+def test_entries_of_other_kernels_are_measured_again(tmp_path, monkeypatch):
+    """A cache file that an earlier version of the kernels wrote (its keys carry no
+    version) does not set the launch shapes of these."""
+    import torch
+    from lh_b200 import Desc, Engine
+    cache = tmp_path / "tune.txt"
+    monkeypatch.setenv("LH_TUNE_CACHE", str(cache))
+    name = torch.cuda.get_device_name().replace("|", "/").replace(" ", "_")
+    cache.write_text(f"{name}|96|96|64 32 4 9 48 2 0.250000\n")
+    e = Engine(Desc(Nx=64, Nz=64, ny=65, dt_mode=1, dt=1e-3))
+    assert e.autotune()["source"] == "measured"
+    assert len(cache.read_text().splitlines()) == 2
+    assert e.autotune()["source"] == "cache"
+    e.close()
