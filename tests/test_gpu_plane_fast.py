@@ -57,3 +57,64 @@ def test_one_cta_planes_are_the_staged_planes(monkeypatch):
             assert np.array_equal(got[f], want[f]), f
         e.close()
     b.close()
+
+
+@pytest.mark.parametrize("Nx,Nz", [(16, 16), (16, 32), (8, 32), (32, 8)])
+def test_one_cta_planes_match_the_generic_and_the_oracle(Nx, Nz, monkeypatch):
+    """The plane shapes that always keep a plane in one CTA and that the sizes above
+    leave out: against the runtime-radix kernels with their bounds, and one step
+    against the oracle with the acceptance bar (1e-12)."""
+    import oracle as O
+    from helpers import oracle_cfg
+    from lh_b200 import Desc, Engine, grids, perturbed_laminar
+    d = Desc(Nx=Nx, Nz=Nz, ny=19, dt_mode=0, CFL=0.5)
+    ic = perturbed_laminar(d, 43, *grids(d))
+    out = []
+    for gen in ("1", "0"):
+        monkeypatch.setenv("LH_GENERIC_FFT", gen)
+        e = Engine(d)
+        e.upload(*ic)
+        e.step(1)
+        e.synchronize()
+        one = e.download()
+        e.step(1)
+        e.synchronize()
+        out.append((e.download(), e.scalars(), one))
+        e.close()
+    for f in ("u1", "u2", "u3", "p"):
+        assert rel_l2(out[1][0][f], out[0][0][f]) <= (1e-12 if f == "p" else 1e-13), f
+    assert abs(out[1][1]["t"] - out[0][1]["t"]) <= 1e-13 * out[0][1]["t"]
+    o = O.Oracle(oracle_cfg(d))
+    o.load_state(*ic)
+    o.step(1)
+    want = o.state()
+    for f in ("u1", "u2", "u3", "p"):
+        assert rel_l2(out[1][2][f], want[f]) <= 1e-12, f
+
+
+@pytest.mark.parametrize("N,ny,mb", [(32, 153, "8"), (32, 66, "6"), (64, 154, "24"), (72, 66, "12"), (128, 153, "48")])
+def test_states_do_not_depend_on_the_staging(N, ny, mb, monkeypatch):
+    """Whatever rounds a staging budget gives -- one, an even number of about the same
+    size, a last one that is shorter -- a plane and its CFL maxima are the same
+    operations: the same bits."""
+    import numpy as np
+    from lh_b200 import Desc, Engine, grids, perturbed_laminar
+    d = Desc(Nx=N, Nz=N, ny=ny, dt_mode=0, CFL=0.5)
+    ic = perturbed_laminar(d, 44, *grids(d))
+    out = []
+    for v in (None, mb):
+        monkeypatch.delenv("LH_STAGING_MB", raising=False)
+        if v:
+            monkeypatch.setenv("LH_STAGING_MB", v)
+        e = Engine(d)
+        e.upload(*ic)
+        rounds = e.profile(1)["x_products"][1]
+        e.upload(*ic)
+        e.step(3)
+        e.synchronize()
+        out.append((e.download(), e.scalars(), rounds))
+        e.close()
+    assert out[0][2] < out[1][2]
+    assert out[0][1] == out[1][1]
+    for f in ("u1", "u2", "u3", "p"):
+        assert np.array_equal(out[0][0][f], out[1][0][f]), f
