@@ -28,16 +28,17 @@ __device__ __forceinline__ double2 cscale(double s, double2 a) { return make_dou
 
 // Helmholtz rows of one grid (solveU's LU_build, tridLU_3D.f90:163-221):
 // row 0 [0, 1, w0], rows 1..n [-beta d1, 1 - beta (d2 + k2), -beta d3],
-// row n+1 [wt, 1, 0]
+// row n+1 [wt, 1, 0].  With beta times a power of two, and that as one, the
+// interior rows come out times it, the same bits otherwise.
 struct HRow {
     double a1, a2, a3;
 };
 __device__ __forceinline__ HRow helm_row(int j, int n, const double *d, double beta, double k2x, double k2z,
-                                         double w0, double wt)
+                                         double w0, double wt, double one = 1.0)
 {
     if (j == 0) return HRow{0.0, 1.0, w0 * 1.0};
     if (j == n + 1) return HRow{wt, 1.0, 0.0};
-    return HRow{-beta * d[3 * j], 1.0 - beta * (d[3 * j + 1] + k2x + k2z), -beta * d[3 * j + 2]};
+    return HRow{-beta * d[3 * j], one - beta * (d[3 * j + 1] + k2x + k2z), -beta * d[3 * j + 2]};
 }
 
 }  // namespace lh

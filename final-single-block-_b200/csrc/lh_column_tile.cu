@@ -184,6 +184,15 @@ __device__ __forceinline__ void mob_rescale(Mob &m)
     m.d *= s;
 }
 
+// The power of two that brings the interior rows of a stiff column to about one, for the
+// products of their maps: at time steps where a row's entries pass 1e34 the product of
+// nine would leave the range of a double, though the recurrence does not.
+__device__ __forceinline__ double helm_scale(double beta, const double *d, double k2x, double k2z)
+{
+    const int e = __double2hiint(fabs(beta) * (fabs(d[4]) + fabs(k2x) + fabs(k2z))) >> 20;
+    return e < 0x3ff || e >= 0x7fe ? 1.0 : __hiloint2double((0x7fe - e) << 20, 0);
+}
+
 // Inverse pivots of the Helmholtz systems of one grid (w.blk: 0 u, 1 v) for
 // kFactorColumns columns: LU_build + LU_dec (tridLU_3D.f90:163-221, 327-364).
 // Bound by the length of the chain, one division a row, so kFactorBlocks lanes
@@ -215,9 +224,10 @@ __global__ void __launch_bounds__(kFactorColumns *kFactorBlocks) k_factors(const
     const int K = (n + L - 1) / L, r0 = min(n + 1, 1 + b * K), r1 = min(n + 1, r0 + K);  // interior rows of the block
     __syncthreads();
     Mob m{1.0, 0.0, 0.0, 1.0};
+    const double sc = helm_scale(beta, sd, k2x, k2z);
 #pragma unroll 1
     for (int j = r0; j < r1; j++) {
-        const HRow h = helm_row(j, n, sd, beta, k2x, k2z, w0, wt);
+        const HRow h = helm_row(j, n, sd, beta * sc, k2x, k2z, w0, wt, sc);
         m = Mob{h.a3 * m.c, h.a3 * m.d, fma(h.a2, m.c, -h.a1 * m.a), fma(h.a2, m.d, -h.a1 * m.b)};
         if (((j - r0) & 7) == 7) mob_rescale(m);
     }
@@ -651,10 +661,11 @@ __global__ void __launch_bounds__(kTileBlocks * 8) k_lusolu_tile(const Inst *__r
     __syncthreads();
     // pivots
     Mob m{1.0, 0.0, 0.0, 1.0};
+    const double sc = helm_scale(beta, sd, k2x, k2z);
 #pragma unroll
     for (int q = 0; q < K; q++) {
         if (r0 + q > n + 1) continue;
-        const HRow h = helm_row(r0 + q, n, sd, beta, k2x, k2z, w0, wt);
+        const HRow h = helm_row(r0 + q, n, sd, beta * sc, k2x, k2z, w0, wt, sc);
         m = Mob{h.a3 * m.c, h.a3 * m.d, fma(h.a2, m.c, -h.a1 * m.a), fma(h.a2, m.d, -h.a1 * m.b)};
     }
     mob_rescale(m);

@@ -103,3 +103,47 @@ def test_profile_counts_the_factors_as_column_pass():
         prof = e.profile(2)
         assert prof["dt"][1] == 2 and prof["column"][1] == 12, prof
         e.close()
+
+
+@pytest.mark.parametrize("ny,dt", [(65, 1e100), (153, 1e80), (257, 1e34), (257, 1e60), (153, 0.0), (257, 1e-300)])
+def test_noalloc_solve_at_extreme_time_steps(ny, dt):
+    """Products of a block's maps stay in range wherever the recurrence does; the bound of
+    the row-limit test."""
+    import numpy as np
+    import torch
+    from lh_b200 import Desc, Engine
+    d = Desc(Nx=32, Nz=18, ny=ny, dt_mode=1, dt=5e-3)
+    e = Engine(d)
+    for grid in (1, 2):
+        n = d.nyu + 2 if grid == 2 else d.nyv + 2
+        rng = np.random.default_rng(ny)
+        rhs = rng.standard_normal((d.ncols, n)) + 1j * rng.standard_normal((d.ncols, n))
+        want = e.lusolu(grid, 2, dt, rhs)
+        x = torch.from_numpy(np.ascontiguousarray(rhs.T)).to("cuda")
+        torch.cuda.synchronize()
+        assert e.L.lh_lusolu_noalloc(e.h, grid, 2, dt, x.data_ptr(), x.data_ptr()) == 0
+        e.synchronize()
+        assert np.isfinite(want).all() and rel_l2(x.cpu().numpy().T, want) <= 1e-13
+    e.close()
+
+
+@pytest.mark.parametrize("N,ny", [(16, 97), (32, 257)])
+@pytest.mark.parametrize("dt", [1e10, 1e45])
+def test_tiles_at_extreme_time_steps(N, ny, dt, monkeypatch):
+    """One substep, whose implicit part is then all there is, against the sequential pass
+    with the acceptance bar of a step (1e-12)."""
+    import numpy as np
+    from lh_b200 import Desc, Engine, grids, perturbed_laminar
+    d = Desc(Nx=N, Nz=N, ny=ny, dt_mode=1, dt=dt)
+    ic = perturbed_laminar(d, 72, *grids(d))
+    out = []
+    for limit in ("0", "1000000000"):
+        monkeypatch.setenv("LH_SMALL_COLUMNS", limit)
+        e = Engine(d)
+        e.upload(*ic)
+        e._ck(e.L.lh_substep(e.h, 1), "substep")
+        e.synchronize()
+        out.append(e.download())
+        e.close()
+    for f in ("u1", "u2", "u3", "p"):
+        assert np.isfinite(out[0][f]).all() and rel_l2(out[1][f], out[0][f]) <= 1e-12, f
