@@ -40,7 +40,6 @@ namespace lh {
 
 constexpr int kTileBlocks = 32;  // row blocks, the lanes that share a column
 
-
 // y -> A + B y with complex A, real B: a block of a forward or back
 // substitution.  N systems side by side; the first two share B when N = 3 (u1
 // and u3 have the same matrix).
@@ -269,10 +268,6 @@ __global__ void __launch_bounds__(kFactorColumns *kFactorBlocks) k_factors(const
     if (r0 <= n && r1 == n + 1) inv[(size_t)(n + 1) * nc] = 1.0 / (1.0 - wt * x);
 }
 
-__device__ __forceinline__ void cp16(void *s, const void *g)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
-}
 __device__ __forceinline__ void cp8(void *s, const void *g)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));

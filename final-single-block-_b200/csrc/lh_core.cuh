@@ -5,8 +5,9 @@
 // double2.  column = kr*(Nx/2+1) + i with kr the spectral z row (0..Nz-1,
 // kz >= 0 first, then kz < 0) and i the x mode (0..Nx/2) -- the reference's
 // np=1 column order (start.f90:964-981) -- so one y-plane is contiguous and
-// x is fastest inside it.  Plane kernels read whole planes; column kernels
-// (one thread per column) read row j of all columns with unit stride.  The
+// x is fastest inside it.  Plane kernels read whole planes; the column kernels
+// (32 columns a warp, or tiles of up to 8) read row j of neighbouring columns with
+// unit stride.  The
 // reference's MPI plane<->column transposes (FOU3D.f90:718-2001) therefore
 // have no counterpart at run time; the only transposes are the host-layout
 // conversions at upload/download.

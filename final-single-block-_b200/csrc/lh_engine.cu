@@ -592,8 +592,8 @@ cudaError_t plan_build(Plan &p, const std::vector<const DevInstance *> &insts, b
         }
         cls_of[q] = (int)(it - classes.begin());
     }
-    // Planes per round: the staging of one round, summed over every instance
-    // of the plan, stays inside the L2 budget so staging never reaches HBM.
+    // Planes per round: the staging of the rounds in flight, summed over every instance
+    // of the plan, stays inside the budget (for batches within L2, see staging_budget).
     const size_t ncls = classes.size();
     std::vector<ClassTiles> tiles(ncls);
     std::vector<const HostSetup *> rep(ncls, nullptr);

@@ -23,9 +23,6 @@
 
 // Launch bounds (max threads, min resident CTAs per SM) each kernel's
 // register allocation is sized for.
-#ifndef LH_FFT_MINB
-#define LH_FFT_MINB 2
-#endif
 #ifndef LH_ZINV_T
 #define LH_ZINV_T 256
 #endif

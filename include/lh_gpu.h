@@ -130,7 +130,10 @@ int lh_get_stream(lh_ctx *ctx, void **stream);
 int lh_autotune(lh_ctx *ctx, int force, int *params);
 /* Runs nsteps RK3 steps launch by launch with CUDA events around every
  * kernel and returns, per kernel class (0 z-inverse, 1 x-products,
- * 2 z-forward, 3 dt, 4 column), the summed milliseconds and launch counts. */
+ * 2 z-forward, 3 dt, 4 column), the summed milliseconds and launch counts.
+ * Small planes, which run all three stages in one kernel, count as class 1;
+ * the LU factors that the column pass of a small plan takes from a kernel of
+ * their own count as class 4. */
 int lh_profile(lh_ctx *ctx, int nsteps, double *ms, int *launches);
 /* max |div| after the last projection (error(), littleharsh.f90:370-409) */
 int lh_error_div(lh_ctx *ctx, double *err);
@@ -257,7 +260,10 @@ typedef struct lh_batch lh_batch;
 int lh_batch_create(size_t hbm_budget, lh_batch **out);
 int lh_batch_destroy(lh_batch *b);
 const char *lh_batch_last_error(const lh_batch *b);
-/* Bytes of device memory one instance of this description needs. */
+/* Bytes of device memory one instance of this description needs: the fields
+ * of a batch's member, and at most those of a context by lh_ctx_create
+ * (beside either: a few MB of work tables, streams and graphs, and what the
+ * diagnostics allocate on first use). */
 size_t lh_instance_bytes(const lh_grid_desc *desc);
 /* Admit an instance (returns its slot id >= 0) with its initial state in
  * the column layout; LH_ENOMEM when the budget is exhausted. */
