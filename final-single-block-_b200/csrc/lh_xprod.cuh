@@ -191,11 +191,11 @@ __device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int rows, bo
         __syncwarp();
         // inverse pass 2, products, forward pass 1 of this lane's row of the matrix.  Lanes
         // left over (N1 = 6, 12) take no part: rows are overwritten here without a barrier,
-        // so nobody but their lanes may read them, and zeros leave the maxima alone.
-        {
+        // so nobody but their lanes may read them.
+        if (on) {
             double2 b[N2];
 #pragma unroll
-            for (int n2 = 0; n2 < N2; n2++) b[n2] = on ? Tr[n2] : make_double2(0.0, 0.0);
+            for (int n2 = 0; n2 < N2; n2++) b[n2] = Tr[n2];
             DFT<N2, +1, NX>::run(b, tw);
             if (pair == 0) {
 #pragma unroll
@@ -222,10 +222,7 @@ __device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int rows, bo
             DFT<N2, -1, NX>::run(b, tw);
             TwStep ts(__ldg(tw + r));
 #pragma unroll
-            for (int n2 = 0; n2 < N2; n2++) {
-                const double2 z = n2 > 0 ? twiddle<-1>(ts.next(), b[n2]) : b[n2];
-                if (on) Tr[n2] = z;
-            }
+            for (int n2 = 0; n2 < N2; n2++) Tr[n2] = n2 > 0 ? twiddle<-1>(ts.next(), b[n2]) : b[n2];
         }
         __syncwarp();
         // forward pass 2, split, scale 1/Mx
@@ -233,13 +230,11 @@ __device__ __forceinline__ void xrow(double2 *T, const double2 *tw, int rows, bo
         for (int g = 0; g < ROUNDS; g++) {
             const Task q(g, lane_row, lane_task, r, on, rows);
             const int m = q.m;
-            // lanes without a task read nothing, those of a row without one their row's
-            // first column
-            const bool reads = PACKED ? q.on : on;
+            // packed lanes without a task read nothing, others a column whose values they drop
             const double2 *const Tm = T + (q.row * RS + (m >= 0 ? m : 0));
             double2 e[N1];
 #pragma unroll
-            for (int k1 = 0; k1 < N1; k1++) e[k1] = reads ? Tm[k1 * LD] : make_double2(0.0, 0.0);
+            for (int k1 = 0; k1 < N1; k1++) e[k1] = !PACKED || q.on ? Tm[k1 * LD] : make_double2(0.0, 0.0);
             DFT<N1, -1, NX>::run(e, tw);
             const double h = 0.5 / NX;
 #pragma unroll
