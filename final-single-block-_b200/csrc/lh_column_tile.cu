@@ -12,8 +12,8 @@
 // boundaries are formed in another order (a few ulp).  The LU factors depend on
 // dt alone, so k_factors forms them beside the plane pass.
 //
-// What bounds it: the dependent chain of one CTA (about 32,000 cycles at 154
-// rows, a third of it the right-hand sides' loads), and a large code run once;
+// What bounds it: the dependent chain of one CTA (about 43,000 cycles at 153 rows and 8
+// columns, a third of its waits on the right-hand sides' loads), and a large code run once;
 // so a lane works on the three systems at once, three independent chains, its
 // next row's loads in flight, and the loops stay rolled (unrolled to 108 KB of
 // code the pass was half again as slow).  Column pass alone, us a substep on

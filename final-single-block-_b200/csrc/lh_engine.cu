@@ -42,7 +42,8 @@ size_t staging_units(int chunk) { return (size_t)(chunk + 2 * kRoundStreams) * 3
 // worth more.  Substep on B200, us, 96 / 150 / 200 / 300 / 500 MB: 128x128x153 357 354
 // 355 351 352, 192x192x257 1502 1478 1467 1452 1442, 256x256x257 2642 2629 2616 2613
 // 2604, 216x216x129 1026 975 971 971 969; an odd number of rounds loses up to 5 %.  It
-// never takes more memory than lh_instance_bytes states (lone_chunk).
+// never takes more memory than lh_instance_bytes states (lone_chunk): 157 MB and 349 us
+// at 128x128x153 (345 with 300), all 300 from 192x192x257 on.
 // Not where the generic plane kernels run, which are slower so: 288x288x65 2408 us at
 // 96 MB, 2496 at 300, 384x384x33 2133 and 2213, 288x96x65 742 and 747.
 size_t staging_budget(bool lone)

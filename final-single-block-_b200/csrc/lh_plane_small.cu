@@ -17,8 +17,9 @@
 // lane reads and writes its own modes only, the face rows first), so only two
 // block barriers separate the three steps.
 //
-// What bounds it: latency at two CTAs an SM (the plane's 78 KB and the row
-// matrices), then the FP64 pipe, 35 % busy.  B200, us a substep, staged -> here:
+// What bounds it: the shared-memory / L1 data pipe, 67 % busy at 16 channels of 32 x
+// 32 x 153, and the FP64 pipe, 44 %, at two CTAs an SM (the plane's 78 KB and the row
+// matrices).  B200, us a substep, staged -> here:
 // 64 channels of 32 x 32 x 153 1515 -> 1239, 16 of them 370 -> 323, 3 of them 92 -> 86, 2
 // 58 -> 63; 16 x 16 x 153 alone 33.7 -> 31.5, x 97 28.0 -> 24.5; 32 x 32 x 153 alone,
 // whose 152 planes leave four SMs with two, 41.3 -> 46.9 (small_plane_pays decides).
