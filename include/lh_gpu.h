@@ -249,7 +249,9 @@ int lh_set_scalars(lh_ctx *ctx, double t, int iter, double mpgx);
  * (cudaGetSymbolAddress), so make it before any stream capture.  Calls are
  * ordered on the context's stream; calls that overlap on the GPU (other
  * streams, other contexts on the same device) share the scratch and race.
- * Every call overwrites the scratch rows it uses before reading them. */
+ * Every call overwrites the scratch rows it uses before reading them.  Up to
+ * 288 rows a column is solved in blocks of rows, so the last bits need not be
+ * those of lh_lusolu. */
 int lh_lusolu_noalloc(lh_ctx *ctx, int grid, int kRK, double dt,
                       const double *rhs_dev, double *u_dev);
 
