@@ -183,13 +183,13 @@ __device__ __forceinline__ void mob_rescale(Mob &m)
     m.d *= s;
 }
 
-// The power of two that brings the interior rows of a stiff column to about one, for the
-// products of their maps: at time steps where a row's entries pass 1e34 the product of
-// nine would leave the range of a double, though the recurrence does not.
+// The power of two that brings the interior rows of a stiff column to about one: at time
+// steps where a row's entries pass 1e30 the product of eight or nine maps would leave
+// the range of a double, though the recurrence does not.  1 otherwise.
 __device__ __forceinline__ double helm_scale(double beta, const double *d, double k2x, double k2z)
 {
     const int e = __double2hiint(fabs(beta) * (fabs(d[4]) + fabs(k2x) + fabs(k2z))) >> 20;
-    return e < 0x3ff || e >= 0x7fe ? 1.0 : __hiloint2double((0x7fe - e) << 20, 0);
+    return e < 0x3ff + 100 || e >= 0x7fe ? 1.0 : __hiloint2double((0x7fe - e) << 20, 0);
 }
 
 // Inverse pivots of the Helmholtz systems of one grid (w.blk: 0 u, 1 v) for
@@ -223,12 +223,13 @@ __global__ void __launch_bounds__(kFactorColumns *kFactorBlocks) k_factors(const
     const int K = (n + L - 1) / L, r0 = min(n + 1, 1 + b * K), r1 = min(n + 1, r0 + K);  // interior rows of the block
     __syncthreads();
     Mob m{1.0, 0.0, 0.0, 1.0};
-    const double sc = helm_scale(beta, sd, k2x, k2z);
+    // stiff columns row by row: times the scale, the rows took 8 more registers (five CTAs an SM)
+    const int every = helm_scale(beta, sd, k2x, k2z) != 1.0 ? 0 : 7;
 #pragma unroll 1
     for (int j = r0; j < r1; j++) {
-        const HRow h = helm_row(j, n, sd, beta * sc, k2x, k2z, w0, wt, sc);
+        const HRow h = helm_row(j, n, sd, beta, k2x, k2z, w0, wt);
         m = Mob{h.a3 * m.c, h.a3 * m.d, fma(h.a2, m.c, -h.a1 * m.a), fma(h.a2, m.d, -h.a1 * m.b)};
-        if (((j - r0) & 7) == 7) mob_rescale(m);
+        if (((j - r0) & every) == every) mob_rescale(m);
     }
     mob_rescale(m);
     maps[t] = m;
